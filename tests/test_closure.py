@@ -2,7 +2,7 @@
 use inside the particle step, and a small end-to-end gain check.
 
 The closure has no counterpart in the reference; the numpy reference
-(oracle/mlp_ref.py) is itself checked against finite differences.
+(oracle/M.py) is itself checked against finite differences.
 Tolerances: GPU gradient vs numpy 1e-4 relative (FP32 vs FP64), inference
 1e-5 relative to the output scale.
 """
@@ -300,3 +300,48 @@ def test_batched_pair_runs_equal_single_runs():
     for cfg, b in zip(cfgs, batched):
         single = closure.run_pair(cfg, 3, 24, 40)
         assert np.array_equal(b[0], single[0])
+
+
+def _numpy_training(w, X, T, epochs, lr, seed):
+    """The trainer's Adam in 64 bits: minibatches of 64 in its epoch order, the step size a half cosine to zero."""
+    w = np.asarray(w, np.float64).copy()
+    n, B = len(X), 64
+    Xs = (X - w[M.OFF["xmu"][0]:][:13]) / w[M.OFF["xsd"][0]:][:13]
+    Ts = (T - w[M.OFF["ymu"][0]:][:12]) / w[M.OFF["ysd"][0]:][:12]
+    m = np.zeros(M.NPARAM)
+    v = np.zeros(M.NPARAM)
+    nb, t, losses = (n + B - 1) // B, 0, []
+    for ep in range(epochs):
+        h = (seed * 2654435761 + ep * 40503 + 12345) % 2 ** 32
+        off, stride = h % n, 1 + (h >> 8) % n
+        while np.gcd(stride, n) != 1:
+            stride = stride % n + 1
+        loss = 0.0
+        for b in range(nb):
+            i = (np.arange(b * B, min(n, b * B + B)) * stride % n + off) % n
+            loss += M.loss_std(w, Xs[i], Ts[i]) * len(i)
+            g = M.grad_std(w, Xs[i], Ts[i])
+            t += 1
+            m = 0.9 * m + 0.1 * g
+            v = 0.999 * v + 0.001 * g * g
+            rate = 0.5 * lr * (1 + np.cos(np.pi * (t - 1) / (epochs * nb)))
+            w[:M.NPARAM] -= rate * (m / (1 - 0.9 ** t)) / (np.sqrt(v / (1 - 0.999 ** t)) + 1e-8)
+        losses.append(loss / n)
+    return w, np.array(losses)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 7, 8, 63, 64, 65, 200])
+def test_gpu_training_follows_numpy_adam(n):
+    """Partial minibatches, idle samples of a CTA and epochs of one or several minibatches.  FP32 sums of at most 64
+    terms are off by a few 1e-7; Adam passes that on relative to each gradient, so two epochs stay well inside 1e-5
+    of the weights' norm."""
+    from lbcuda_b200 import closure
+    rng = np.random.default_rng(n)
+    X = rng.normal(size=(n, 13)).astype(np.float32)
+    T = rng.normal(size=(n, 12)).astype(np.float32)
+    w0 = closure.init_weights(rng.normal(size=(50, 13)), rng.normal(size=(50, 12)), seed=3)
+    w, loss = closure.train(X, T, epochs=2, lr=2e-3, seed=5, w=w0.copy())
+    ref, rloss = _numpy_training(w0, X, T, 2, float(np.float32(2e-3)), 5)
+    assert np.linalg.norm(w - ref) <= 1e-5 * np.linalg.norm(ref)
+    assert np.abs(loss - rloss).max() <= 1e-5 * np.abs(rloss).max()
