@@ -33,9 +33,9 @@
 #include "lbx_closure.h"
 
 #include <cooperative_groups.h>
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
-#include <vector>
 
 namespace lbx {
 
@@ -360,6 +360,17 @@ __global__ void __cluster_dims__(NCL, 1, 1) __launch_bounds__(TT) k_mlp_train(Tr
     for (int j = tid; j < NC4; j += TT) *reinterpret_cast<float4*>(a.w + 4 * j) = ld4(sm + chunk_at(j));
 }
 
+// Raw features or targets (rows of D) standardised in place with the blob's
+// mean and std: the two roundings of the host loop this replaces (0.45 ms of
+// a 15 ms call at 30,976 samples)
+__global__ void k_standardise(float* __restrict__ v, size_t n, int D, const float* __restrict__ mean,
+                              const float* __restrict__ sd) {
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
+    const int k = int(i % unsigned(D));
+    v[i] = (v[i] - mean[k]) / sd[k];
+  }
+}
+
 // ---------------------------------------------------------------------------
 // inference: one warp per sample, weights (and normalisation) in shared memory
 // ---------------------------------------------------------------------------
@@ -445,13 +456,16 @@ int lbx_closure_train(float* weights, const float* X, const float* T, int32_t n,
   const size_t nx = size_t(n) * lbx::DIN, nt = size_t(n) * lbx::DOUT;
   Dev dX(nx * 4), dT(nt * 4), dW(size_t(L::TOTAL) * 4), dL(size_t(epochs) * 4);
   if (!dX.p || !dT.p || !dW.p || !dL.p) return LBX_ERR_ALLOC;
-  // standardise with the statistics stored in the blob
-  std::vector<float> Xs(nx), Ts(nt);
-  for (size_t i = 0; i < nx; ++i) Xs[i] = (X[i] - weights[L::XMU + i % lbx::DIN]) / weights[L::XSD + i % lbx::DIN];
-  for (size_t i = 0; i < nt; ++i) Ts[i] = (T[i] - weights[L::YMU + i % lbx::DOUT]) / weights[L::YSD + i % lbx::DOUT];
-  int rc = rc_of(cudaMemcpy(dX.p, Xs.data(), nx * 4, cudaMemcpyHostToDevice));
-  if (!rc) rc = rc_of(cudaMemcpy(dT.p, Ts.data(), nt * 4, cudaMemcpyHostToDevice));
+  int rc = rc_of(cudaMemcpy(dX.p, X, nx * 4, cudaMemcpyHostToDevice));
+  if (!rc) rc = rc_of(cudaMemcpy(dT.p, T, nt * 4, cudaMemcpyHostToDevice));
   if (!rc) rc = rc_of(cudaMemcpy(dW.p, weights, size_t(L::TOTAL) * 4, cudaMemcpyHostToDevice));
+  if (!rc) {
+    float *x = (float*)dX.p, *t = (float*)dT.p, *w = (float*)dW.p;
+    const int bx = int(std::min<size_t>((nx + 255) / 256, 1184)), bt = int(std::min<size_t>((nt + 255) / 256, 1184));
+    lbx::k_standardise<<<bx, 256>>>(x, nx, lbx::DIN, w + L::XMU, w + L::XSD);
+    lbx::k_standardise<<<bt, 256>>>(t, nt, lbx::DOUT, w + L::YMU, w + L::YSD);
+    rc = rc_of(cudaGetLastError());
+  }
   if (rc) return rc;
   lbx::TrainArgs a{(const float*)dX.p, (const float*)dT.p, n, (float*)dW.p, (float*)dL.p, nullptr, epochs, lr,
                    0.9f, 0.999f, 1e-8f, unsigned(seed)};
