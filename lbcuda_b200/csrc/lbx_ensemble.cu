@@ -6,8 +6,8 @@
 // ensemble forks from the ensemble stream to the stream of every box with
 // spheres, runs that box's sphere pre-kernels there, joins, launches ONE
 // persistent colour-gradient kernel for the fluid of all boxes
-// (k_cg_lean_multi: CTAs take (box, column, z-segment) work items, longest
-// first) on the ensemble stream, then forks and joins again around the sphere
+// (k_cg_lean2_multi for 16-bit storage, else k_cg_lean_multi: CTAs take (box,
+// column, z-segment) work items, longest first) on the ensemble stream, then forks and joins again around the sphere
 // post-kernels.  The boxes' small sphere kernels thus run side by side
 // instead of one after the other.  Two consecutive steps (the ping-pong
 // parity) are captured once into a CUDA graph (the forks become parallel

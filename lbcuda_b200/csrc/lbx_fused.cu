@@ -30,6 +30,10 @@
 // ring and the two boundary planes of each segment.  The particle variant
 // (PART) also copies each cell's flag words and side phase field with its
 // pulls and collides only fluid cells.
+//
+// 16-bit boxes without spheres and the ensemble run the same march with two
+// cells per thread and two roles per CTA (phase_column2 and
+// collide_column2 below); the results are the same bits.
 #include "lbx_device.cuh"
 
 #include <algorithm>
@@ -1287,6 +1291,576 @@ __global__ void __launch_bounds__(TX* TY, MINB)
 }
 
 // ---------------------------------------------------------------------------
+// Two cells per thread (16-bit storage, box staging)
+// ---------------------------------------------------------------------------
+// The column march of lean_column for 16-bit pairs staged in boxes, with the
+// two halves of every packed FP32 instruction holding two CELLS instead of a
+// direction and its opposite.  The whole collision is then packed, not only
+// its per-direction part: momentum, gradient, coefficients and the equilibrium
+// run once per two cells, no value is moved to form or split a pair, and a
+// store's address serves both cells.  Each lane performs the roundings of
+// lean_column in the same order, so both give the same bits.
+//
+// Thread (warp w, lane = 16 h + c) owns the cells (x0 + c, y) and
+// (x0 + 16 + c, y) of row y0 + 4 (w / 2) + w % 2 + 2 h: the second cell is a
+// constant 16 cells on in shared and global memory, and the two rows of a
+// warp lie 2 x 40 words apart in a box, half the banks, so its reads do not
+// conflict.
+using V2 = float2;
+__device__ __forceinline__ V2 v2(float a) { return make_float2(a, a); }
+// a - b (the product with -1 is exact: one rounding)
+__device__ __forceinline__ V2 v_sub(V2 a, V2 b) { return p_fma(b, v2(-1.f), a); }
+
+// e_l . (a0, a1, a2) of an odd direction l (its last component is positive)
+__device__ __forceinline__ V2 v_edot(int l, const V2 a[3]) {
+  const int e[3] = {ex(l), ey(l), ez(l)};
+  const int j = e[2] ? 2 : (e[1] ? 1 : 0);  // last component
+  V2 r = a[j];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (i < j && e[i]) r = e[i] > 0 ? p_add(a[i], r) : v_sub(r, a[i]);
+  return r;
+}
+
+// the BGK half of relax_sums for two cells, up to the per-direction values,
+// which recolour2 forms where it uses them (relaxed2)
+struct Relaxed2 {
+  V2 u, v, w, c0, omega, omm, inv, ors;
+};
+
+__device__ __forceinline__ Relaxed2 relax2(const LeanConst<float>& K, const V2 S[Q], V2 rR, V2 rB) {
+  Relaxed2 X;
+  const V2 rs = p_add(rR, rB);
+  if (K.omega >= 0.f) {
+    X.omega = v2(K.omega);
+  } else {
+    auto om = [&](float r, float b, float t) {
+      const float ph = (r - b) / t;
+      const float visc = 1.f / (0.5f * (1.f + ph) * K.inv_viscR + 0.5f * (1.f - ph) * K.inv_viscB);
+      return 1.f / fm(visc, K.inv_cssq, 0.5f);
+    };
+    X.omega = make_float2(om(rR.x, rB.x, rs.x), om(rR.y, rB.y, rs.y));
+  }
+  X.omm = v_sub(v2(1.f), X.omega);
+  X.inv = make_float2(rcp_c(rs.x), rcp_c(rs.y));
+  V2 mu = v2(0.f), mv = v2(0.f), mw = v2(0.f);
+#pragma unroll
+  for (int p = 1; p <= 9; ++p) {
+    const int l = 2 * p - 1;
+    const V2 d = v_sub(S[l], S[l + 1]);
+    if (ex(l)) mu = ex(l) > 0 ? p_add(mu, d) : v_sub(mu, d);
+    if (ey(l)) mv = ey(l) > 0 ? p_add(mv, d) : v_sub(mv, d);
+    if (ez(l)) mw = ez(l) > 0 ? p_add(mw, d) : v_sub(mw, d);
+  }
+  X.u = p_mul(X.inv, mu);
+  X.v = p_mul(X.inv, mv);
+  X.w = p_mul(X.inv, mw);
+  X.c0 = p_fma(v2(-1.5f), p_fma(X.u, X.u, p_fma(X.v, X.v, p_mul(X.w, X.w))), v2(1.f));
+  X.ors = p_mul(X.omega, rs);
+  return X;
+}
+
+// recolour_sums for two cells with a colour gradient (px, py, pz, |psi|^2 =
+// psq): out(l, a, b) takes the post-collision pairs, a = first halves of the
+// two cells, b = second halves.  S: the stored sums per direction.
+template <bool SD, typename O>
+__device__ __forceinline__ void recolour2(const LeanConst<float>& K, const Relaxed2& X, const V2 S[Q], V2 rR, V2 rB,
+                                          V2 px, V2 py, V2 pz, V2 psq, O&& out) {
+  // relaxed sums: h_l = omm S_l + (omega rho w_l A_l(u) + omm s_l)
+  V2 kc[3], hs[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    kc[k] = p_mul(X.ors, v2(K.w[k]));
+    hs[k] = p_mul(X.omm, v2(K.s[0][k] + K.s[1][k]));
+  }
+  const V2 uu[3] = {X.u, X.v, X.w};
+  auto relaxed_pair = [&](int l, V2& ha, V2& hb) {  // directions l (odd) and l + 1
+    const int k = wclass(l);
+    const V2 eu = v_edot(l, uu);
+    const V2 P = p_fma(p_mul(v2(4.5f), eu), eu, X.c0);
+    ha = p_fma(X.omm, S[l], p_fma(kc[k], p_fma(v2(3.f), eu, P), hs[k]));
+    hb = p_fma(X.omm, S[l + 1], p_fma(kc[k], p_fma(v2(-3.f), eu, P), hs[k]));
+  };
+  const V2 h0 = p_fma(X.omm, S[0], p_fma(kc[0], X.c0, hs[0]));
+  const V2 ipn = make_float2(rsqrt_c(psq.x), rsqrt_c(psq.y));
+  const V2 pn = p_mul(psq, ipn);
+  const V2 ac = p_mul(p_mul(v2(9.f / 4.f), X.omega), v2(K.sigma));
+  const V2 coef = p_mul(p_mul(p_mul(p_mul(v2(K.beta), rR), rB), X.inv), ipn);
+  const V2 kR = p_mul(rR, X.inv), kB = p_mul(rB, X.inv);
+  V2 K1[3], nK0[3], K3[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    K1[k] = p_mul(p_mul(ac, v2(K.w[k])), ipn);
+    nK0[k] = p_mul(p_mul(ac, pn), v2(-K.b[k]));
+  }
+  // added, not multiplied, below: formed by scalar products, which (unlike the
+  // packed ones) -fmad=false keeps the compiler from fusing with that sum
+  nK0[0] = make_float2(ac.x * pn.x * -K.b[0], ac.y * pn.y * -K.b[0]);
+  K3[0] = v2(0.f);
+  K3[1] = p_mul(coef, v2(K.w[1]));
+  K3[2] = p_mul(coef, v2(K.w2_sqrt2));
+  const V2 pp3[3] = {px, py, pz};
+  const V2 f0 = p_add(h0, nK0[0]);
+  if constexpr (SD) {
+    const V2 kD = v_sub(kR, kB);
+    out(0, p_add(f0, v2(-K.ssd[0][0])), p_fma(kD, f0, v2(-K.ssd[1][0])));
+    const V2 T2[3] = {v2(0.f), p_mul(v2(2.f), K3[1]), p_mul(v2(2.f), K3[2])};
+    const V2 nT2[3] = {v2(0.f), p_mul(v2(-2.f), K3[1]), p_mul(v2(-2.f), K3[2])};
+#pragma unroll
+    for (int p = 1; p <= 9; ++p) {
+      const int l = 2 * p - 1, k = wclass(l);
+      const V2 ed = v_edot(l, pp3);
+      const V2 pert = p_fma(K1[k], p_mul(ed, ed), nK0[k]);
+      const V2 sS = v2(-K.ssd[0][k]), sD = v2(-K.ssd[1][k]);
+      V2 ha, hb;
+      relaxed_pair(l, ha, hb);
+      const V2 fa = p_add(ha, pert), fb = p_add(hb, pert);
+      out(l, p_add(fa, sS), p_fma(kD, fa, p_fma(T2[k], ed, sD)));
+      out(l + 1, p_add(fb, sS), p_fma(kD, fb, p_fma(nT2[k], ed, sD)));
+    }
+  } else {
+    out(0, p_fma(f0, kR, v2(-K.s[0][0])), p_fma(f0, kB, v2(-K.s[1][0])));
+#pragma unroll
+    for (int p = 1; p <= 9; ++p) {
+      const int l = 2 * p - 1, k = wclass(l);
+      const V2 ed = v_edot(l, pp3);
+      const V2 pert = p_fma(K1[k], p_mul(ed, ed), nK0[k]);
+      const V2 T = p_mul(K3[k], ed);
+      const V2 sR = v2(-K.s[0][k]), sB = v2(-K.s[1][k]);
+      V2 ha, hb;
+      relaxed_pair(l, ha, hb);
+      const V2 fa = p_add(ha, pert), fb = p_add(hb, pert);
+      out(l, p_fma(kR, fa, p_add(T, sR)), p_fma(kB, fa, v_sub(sB, T)));
+      out(l + 1, p_fma(kR, fb, v_sub(sR, T)), p_fma(kB, fb, p_add(T, sB)));
+    }
+  }
+}
+
+// bgk_components for two cells: in(l, a, b) gives the pulled pairs (stored
+// form) as out() takes them
+template <bool SD, typename I, typename O>
+__device__ __forceinline__ void bgk2(const LeanConst<float>& K, const Relaxed2& X, V2 rA, V2 rB, I&& in, O&& out) {
+  const float(&sh)[2][3] = SD ? K.ssd : K.s;
+  const V2 omm = v_sub(v2(1.f), X.omega);
+  const V2 oA = p_mul(X.omega, rA), oB = p_mul(X.omega, rB);
+  const V2 uu[3] = {X.u, X.v, X.w};
+  auto one = [&](int l, V2 A) {
+    const int k = wclass(l);
+    V2 a, b;
+    in(l, a, b);
+    out(l, p_fma(a, omm, p_fma(p_mul(oA, v2(K.w[k])), A, p_mul(X.omega, v2(-sh[0][k])))),
+        p_fma(b, omm, p_fma(p_mul(oB, v2(K.w[k])), A, p_mul(X.omega, v2(-sh[1][k])))));
+  };
+  one(0, X.c0);
+#pragma unroll
+  for (int p = 1; p <= 9; ++p) {
+    const int l = 2 * p - 1;
+    const V2 eu = v_edot(l, uu);
+    const V2 P = p_fma(p_mul(v2(4.5f), eu), eu, X.c0);
+    one(l, p_fma(v2(3.f), eu, P));
+    one(l + 1, p_fma(v2(-3.f), eu, P));
+  }
+}
+
+struct PlaneGrad2 {
+  V2 gx, gy, m;
+};
+
+// plane_grad of the cells at own and own + 16 (row stride WR)
+template <int WR>
+__device__ __forceinline__ PlaneGrad2 plane_grad2(const float* plane, int own) {
+  const V2 W0 = v2(2.f / 3.f), W1 = v2(1.f / 6.f);
+  const float* r0 = plane + own;
+  auto at = [&](int o) { return make_float2(r0[o], r0[o + 16]); };
+  const V2 a = at(-WR - 1), b = at(-WR), c = at(-WR + 1);
+  const V2 d = at(-1), e = at(0), f = at(1);
+  const V2 g = at(WR - 1), h = at(WR), i = at(WR + 1);
+  PlaneGrad2 G;
+  G.gx = p_fma(W0, v_sub(f, d), p_mul(W1, p_add(v_sub(c, a), v_sub(i, g))));
+  G.gy = p_fma(W0, v_sub(h, b), p_mul(W1, p_add(v_sub(g, a), v_sub(i, c))));
+  const V2 lo = p_fma(W0, b, p_mul(W1, p_add(a, c))), mid = p_fma(W0, e, p_mul(W1, p_add(d, f))),
+           hi = p_fma(W0, h, p_mul(W1, p_add(g, i)));
+  G.m = p_fma(W0, mid, p_mul(W1, p_add(lo, hi)));
+  return G;
+}
+
+// Boxes of a column of 32 x TY cells (see the head of this file): per plane
+// and direction l, the rows y0 - 1 - e_ly .. y0 + TY - e_ly and the columns
+// x0 - 4 .. x0 + 35 of direction plane l at z - e_lz, copied by 16-byte
+// cp.async granules (a granule starts on a multiple of 4 cells, so with
+// nx % 4 == 0 the periodic wrap moves whole granules).  Own cell (tx, ty)
+// finds its pull of direction l at box row ty + 1, column tx + 4 - e_lx; ring
+// cell (rx, ry) at row ry, column rx + 3 - e_lx.  Each plane slot has a FULL
+// barrier (every thread arrives once its copies have landed,
+// cp.async.mbarrier.arrive) and an EMPTY barrier (every thread arrives after
+// its last read of the plane), since a thread reads what other threads copied.
+// With spheres also the flag bytes of this and of the previous step (8-byte
+// granules, columns x0 - 8 .. x0 + 39; a box with spheres has nx % 8 == 0) and
+// the side phase field (the pull box's rows and columns, e = 0).
+template <typename S, int TY, bool PART>
+struct Col2 {
+  using R = typename SPair<S>::R;
+  static constexpr int TX = 32, NT = 16 * TY, D = 3;         // NT: threads of each role
+  static constexpr int WR = 40, CELLS = WR * (TY + 2);
+  static constexpr int WIN = D;  // window planes
+  static constexpr int BW = 40, ROWS = TY + 2, ELEMS = BW * ROWS, GR = BW / 4, POS = ROWS * GR;
+  static constexpr int FBW = 48, FGR = FBW / 8, FB = ROWS * FBW, FPOS = 2 * ROWS * FGR;
+  static constexpr int RN = Ring<TX, TY>::N;
+  static_assert(sizeof(R) == 4 && POS <= NT && FPOS <= NT && RN <= NT, "one granule per thread");
+  static constexpr size_t PHI = sizeof(float) * WIN * CELLS;
+  static constexpr size_t STAGE = sizeof(R) * D * Q * ELEMS;
+  static constexpr size_t SIDE = PART ? size_t(D) * (2 * FB + sizeof(float) * ELEMS) : 0;
+  static constexpr size_t DENS = sizeof(float4) * D * NT;              // densities of each thread's two cells
+  static constexpr size_t BYTES = PHI + STAGE + SIDE + DENS + 8 * (3 * D + 1);
+  static_assert(PHI % 16 == 0 && STAGE % 16 == 0 && SIDE % 16 == 0, "alignment");
+  static __device__ __forceinline__ float4* dens(unsigned char* b) {
+    return reinterpret_cast<float4*>(b + PHI + STAGE + SIDE);
+  }
+  static __device__ __forceinline__ unsigned long long* bar(unsigned char* b) {
+    return reinterpret_cast<unsigned long long*>(b + PHI + STAGE + SIDE + DENS);
+  }
+  static __device__ __forceinline__ void init(unsigned char* b) {
+    if (threadIdx.x == 0)
+      for (int q = 0; q < 3 * D; ++q) mbar_init(bar(b) + q, NT);
+  }
+};
+
+// Threads of a CTA in two roles, NT of each, that meet only at the barriers of
+// the three stage slots.  The planes a CTA goes through (z0 - 1 .. zend of each
+// of its columns) take the slots in turn:
+//   phase warps (the upper half of the CTA) copy the next plane into its slot
+//     once the collision has left it (EMPTY); when a plane has landed (FULL)
+//     they sum its pulls, write the phase field of the column and its ring
+//     into the window and the densities into the slot's mailbox, and arrive at
+//     the slot's READY barrier;
+//   collision warps (the lower half) take the sums of plane z from the stage
+//     and its densities from the mailbox and leave the slot at once, wait for
+//     plane z + 1 (READY), form the gradient, collide and store.
+// Bound by the bytes in flight: with one plane of a column in flight and one
+// waiting for its collision the kernel took the same 82 us at FP16 128^3 with
+// 745 or 541 instructions per cell, and its copies and stores alone took 85.
+// Two planes of 30 KB in flight per CTA (the slot is released when the
+// collision starts, the next copies start before a plane is awaited):
+// 76.5 us, and 530 against 596 us at 256^3.
+// Order between the roles: plane i of the sequence is copied and summed only
+// after EMPTY of plane i - 3, so its stage, mailbox and window slots are no longer
+// read.
+struct SlotSeq {
+  int q = 0;         // slot of the next plane
+  unsigned par = 0;  // parity of its barriers' phase
+  __device__ __forceinline__ void next() {
+    if (++q == 3) {
+      q = 0;
+      par ^= 1u;
+    }
+  }
+};
+struct PhaseSync {
+  SlotSeq copy, sum;
+};
+
+template <typename S, int TY, bool PART, bool SD>
+__device__ __forceinline__ void phase_column2(const S* __restrict__ A, const Geom& g, const LeanConst<float>& K, int x0,
+                                              int y0, int z0, int zend, unsigned long long* err, int64_t step,
+                                              const LeanPart<float>& PT, unsigned char* smem, PhaseSync& sy) {
+  using M = Col2<S, TY, PART>;
+  using R = typename SPair<S>::R;
+  using RG = Ring<32, TY>;
+  constexpr int D = M::D, WR = M::WR;
+  const bool parts = PART && PT.fnew != nullptr;  // a box of the ensemble may have no spheres
+  float(*const sphi)[M::CELLS] = reinterpret_cast<float(*)[M::CELLS]>(smem);
+  R* const stage = reinterpret_cast<R*>(smem + M::PHI);
+  unsigned char* const fbox = smem + M::PHI + M::STAGE;                            // flags [D][2][FB]
+  float* const pbox = reinterpret_cast<float*>(fbox + D * 2 * M::FB);              // side phase field [D][ELEMS]
+  float4* const dens = M::dens(smem);
+  unsigned long long* const fullb = M::bar(smem);
+  unsigned long long* const emptyb = fullb + D;
+  unsigned long long* const readyb = emptyb + D;
+
+  const int tid = threadIdx.x - M::NT, c = tid & 15, h = (tid >> 4) & 1, wp = tid >> 5;
+  const int ty = 4 * (wp >> 1) + (wp & 1) + 2 * h;
+  const bool row_in = y0 + ty < g.ny;
+  const bool act0 = row_in && x0 + c < g.nx, act1 = row_in && x0 + 16 + c < g.nx;
+  const int own = (ty + 1) * WR + c + 1;
+  const int obase = (ty + 1) * M::BW + c + 4;
+  const int ofb = (ty + 1) * M::FBW + c + 8;
+  // ring cell of this thread (threads 0 .. N-1)
+  int rx = 0, ry = 0;
+  const bool ringer = tid < RG::N;
+  if (tid < RG::RX) { rx = tid; ry = 0; }
+  else if (tid < 2 * RG::RX) { rx = tid - RG::RX; ry = RG::RY - 1; }
+  else if (tid < 2 * RG::RX + TY) { rx = 0; ry = 1 + tid - 2 * RG::RX; }
+  else if (ringer) { rx = RG::RX - 1; ry = 1 + tid - 2 * RG::RX - TY; }
+  const int rslot = ry * WR + rx, rbase = ry * M::BW + rx + 3, rfb = ry * M::FBW + rx + 7;
+  const Planes<const S> Ap{A, 2 * g.n};
+  const unsigned plane_cells = unsigned(g.nx) * unsigned(g.ny);
+  const unsigned cell_xy = unsigned(x0 + c) + unsigned(g.nx) * unsigned(y0 + ty);  // own cell of plane 0
+
+  // granule of this thread (the last POS threads; the ring sits on the first
+  // ones): box row crow, granule ccol of every direction; first cell in its
+  // plane for e_ly = +1, 0, -1
+  const int cpos = tid - (M::NT - M::POS);
+  const bool copier = cpos >= 0;
+  const int crow = copier ? cpos / M::GR : 0, ccol = copier ? cpos - crow * M::GR : 0;
+  unsigned cyx[3] = {0, 0, 0}, fyx = 0;
+  if (copier) {
+    const int cxg = wrap0(x0 - 4 + 4 * ccol, g.nx);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) cyx[k] = unsigned(wrap0(y0 - 2 + k + crow, g.ny) * g.nx + cxg);  // k = 1 - e_ly
+  }
+  // flag granule of this thread: array (this step, previous step), row, 8 cells
+  const int farr = tid / (M::ROWS * M::FGR), frem = tid - farr * (M::ROWS * M::FGR);
+  const int frow = frem / M::FGR, fgr = frem - frow * M::FGR;
+  if constexpr (PART)
+    if (tid < M::FPOS) fyx = unsigned(wrap0(y0 - 1 + frow, g.ny) * g.nx + wrap0(x0 - 8 + 8 * fgr, g.nx));
+
+  // start the copies of plane p into the next slot
+  auto issue = [&](int p) {
+    const int q = sy.copy.q;
+    if (!mbar_wait(emptyb + q, sy.copy.par ^ 1u)) raise_error(err, LBX_DEV_WAIT_TIMEOUT, step, -3);
+    sy.copy.next();
+    unsigned zo[3];  // plane offsets for e_lz = +1, 0, -1
+#pragma unroll
+    for (int k = 0; k < 3; ++k) zo[k] = unsigned(wrap_plane(p - (1 - k), g.nz)) * plane_cells;
+    if (copier) {
+      R* const dst = stage + q * (Q * M::ELEMS) + crow * M::BW + 4 * ccol;
+      auto one = [&](auto lc) {
+        constexpr int l = decltype(lc)::value;
+        cp_async16(dst + l * M::ELEMS, Ap.at(l, int(zo[1 - ez(l)] + cyx[1 - ey(l)])));
+      };
+      unroll_even(one);
+      unroll_odd(one);
+      const int at = q * M::ELEMS + crow * M::BW + 4 * ccol;
+      if constexpr (PART)
+        if (parts) cp_async16(pbox + at, PT.phi + size_t(zo[1] + cyx[1]));
+    }
+    if constexpr (PART)
+      if (parts && tid < M::FPOS)
+        cp_async8(fbox + (q * 2 + farr) * M::FB + frow * M::FBW + 8 * fgr,
+                  (farr ? PT.fold : PT.fnew) + size_t(zo[1] + fyx));
+    mbar_arrive_cp_async(fullb + q);
+  };
+
+  // Phase field (and clamped densities) of one staged cell, the values of
+  // lean_column's cell_phase without its branches, so that the sums of the own
+  // cells and of the ring cell are one block of independent chains: e = the
+  // cell's element in a box, f = its flag byte, owns: the CTA collides it
+  auto cell_phase = [&](int q, int e, int f, unsigned cell, bool owns, float& rR, float& rB) -> float {
+    const R* const st = stage + q * (Q * M::ELEMS) + e;
+    stage_rho<S, float, SD>([&](int l) { return st[l * M::ELEMS - ex(l)]; }, K, rR, rB);
+    bool fluid = true;
+    int8_t fn = LBX_FLUID_FLUID;
+    if constexpr (PART) {
+      if (parts) {
+        fn = int8_t(fbox[q * 2 * M::FB + f]);
+        fluid = fn == LBX_FLUID_FLUID && int8_t(fbox[(q * 2 + 1) * M::FB + f]) == LBX_FLUID_FLUID;
+      }
+    }
+    if (owns && fluid && (rR < -10.f || rR > 10.f || rB < -10.f || rB > 10.f))
+      raise_error(err, LBX_DEV_RHO_RANGE, step, cell);
+    rR = clamp0(rR);
+    rB = clamp0(rB);
+    if constexpr (PART) {
+      if (!fluid) rR = rB = 0.f;
+      float ph = phase_of(rR, rB);
+      // surface cells and new fluid cells: the side phase field
+      if (!fluid && (fn == LBX_FLUID_SPHERELIST || fn == LBX_FLUID_FLUID)) ph = pbox[q * M::ELEMS + e];
+      if (owns && !fluid && fn == LBX_FLUID_FLUID) {  // new fluid cell: interleaved densities
+        rR = PT.rhoR[2 * size_t(cell)];
+        rB = PT.rhoB[2 * size_t(cell)];
+      }
+      return ph;
+    }
+    return phase_of(rR, rB);
+  };
+
+  issue(z0 - 1);
+  issue(z0);
+  for (int p = z0 - 1; p <= zend; ++p) {
+    if (p > z0 - 1 && p + 1 <= zend) issue(p + 1);  // in flight beside plane p
+    const int q = sy.sum.q;
+    if (!mbar_wait(fullb + q, sy.sum.par)) raise_error(err, LBX_DEV_WAIT_TIMEOUT, step, -2);
+    sy.sum.next();
+    const bool in = p >= z0 && p < zend;
+    const unsigned cell = cell_xy + unsigned(in ? p : z0) * plane_cells;
+    float* const win = sphi[q];
+    float4 r;
+    float qR, qB;
+    const float pa = cell_phase(q, obase, ofb, cell, in && act0, r.x, r.y);
+    const float pb = cell_phase(q, obase + 16, ofb + 16, cell + 16, in && act1, r.z, r.w);
+    const float pr = cell_phase(q, rbase, rfb, 0u, false, qR, qB);
+    win[own] = pa;
+    win[own + 16] = pb;
+    if (ringer) win[rslot] = pr;
+    dens[q * M::NT + tid] = r;
+    mbar_arrive(readyb + q);
+  }
+}
+
+template <typename S, int TY, bool PART, bool SD>
+__device__ __forceinline__ void collide_column2(const S* __restrict__ A, S* __restrict__ B, const Geom& g,
+                                                const LeanConst<float>& K, int x0, int y0,
+                                                int z0, int zend, unsigned long long* err, int64_t step,
+                                                bool parts, unsigned char* smem, SlotSeq& sy) {
+  using M = Col2<S, TY, PART>;
+  using R = typename SPair<S>::R;
+  constexpr int D = M::D, WR = M::WR;
+  float(*const sphi)[M::CELLS] = reinterpret_cast<float(*)[M::CELLS]>(smem);
+  R* const stage = reinterpret_cast<R*>(smem + M::PHI);
+  unsigned char* const fbox = smem + M::PHI + M::STAGE;
+  const float4* const dens = M::dens(smem);
+  unsigned long long* const emptyb = M::bar(smem) + D;
+  unsigned long long* const readyb = emptyb + D;
+  const int tid = threadIdx.x, c = tid & 15, h = (tid >> 4) & 1, wp = tid >> 5;
+  const int ty = 4 * (wp >> 1) + (wp & 1) + 2 * h;
+  const bool row_in = y0 + ty < g.ny;
+  const bool act0 = row_in && x0 + c < g.nx, act1 = row_in && x0 + 16 + c < g.nx;
+  const int own = (ty + 1) * WR + c + 1;
+  const int obase = (ty + 1) * M::BW + c + 4;
+  const int ofb = (ty + 1) * M::FBW + c + 8;
+  const Planes<const S> Ap{A, 2 * g.n};
+  const Planes<S> Bp{B, 2 * g.n};
+  const unsigned plane_cells = unsigned(g.nx) * unsigned(g.ny);
+  const unsigned cell_xy = unsigned(x0 + c) + unsigned(g.nx) * unsigned(y0 + ty);
+
+  // the next plane's slot (stage, mailbox and window), once READY
+  auto ready_wait = [&]() -> int {
+    const int q = sy.q;
+    if (!mbar_wait(readyb + q, sy.par)) raise_error(err, LBX_DEV_WAIT_TIMEOUT, step, -1);
+    sy.next();
+    return q;
+  };
+  const int qm = ready_wait();
+  PlaneGrad2 gm = plane_grad2<WR>(sphi[qm], own);
+  mbar_arrive(emptyb + qm);
+  int qz = ready_wait();  // slot of plane z
+  PlaneGrad2 g0 = plane_grad2<WR>(sphi[qz], own);
+  bool was_off = false;  // of this warp
+  for (int z = z0; z < zend; ++z) {
+    bool col0 = act0, col1 = act1;
+    if constexpr (PART) {
+      if (parts) {
+        col0 = act0 && int8_t(fbox[qz * 2 * M::FB + ofb]) == LBX_FLUID_FLUID;
+        col1 = act1 && int8_t(fbox[qz * 2 * M::FB + ofb + 16]) == LBX_FLUID_FLUID;
+      }
+    }
+    const float4 r = dens[qz * M::NT + tid];
+    const V2 rRc = make_float2(r.x, r.z), rBc = make_float2(r.y, r.w);
+    const unsigned cell = cell_xy + unsigned(z) * plane_cells;
+    const R* const zb = stage + qz * (Q * M::ELEMS) + obase;
+    auto staged0 = [&](int l) -> R { return zb[l * M::ELEMS - ex(l)]; };
+    auto staged1 = [&](int l) -> R { return zb[l * M::ELEMS - ex(l) + 16]; };
+    if constexpr (PART) {  // a solid cell keeps the plain pull
+      const bool s0 = act0 && !col0, s1 = act1 && !col1;
+      if (s0 || s1) {
+#pragma unroll
+        for (int l = 0; l < Q; ++l) {
+          S* const at = Bp.at(l, int(cell));
+          if (s0) *reinterpret_cast<R*>(at) = staged0(l);
+          if (s1) *reinterpret_cast<R*>(at + 32) = staged1(l);
+        }
+      }
+    }
+    V2 Ss[Q];
+#pragma unroll
+    for (int l = 0; l < Q; ++l)
+      Ss[l] = SD ? make_float2(SPair<S>::first(staged0(l)), SPair<S>::first(staged1(l)))
+                 : make_float2(SPair<S>::sum(staged0(l)), SPair<S>::sum(staged1(l)));
+    // The slot is free: only a cell without a gradient needs more than the
+    // sums.  A warp that met such a cell in the plane before (the bulk of one
+    // fluid) keeps the slot until its cells are done, otherwise they are
+    // pulled again from L2.
+    const bool keep = was_off;
+    if (!keep) mbar_arrive(emptyb + qz);
+    const Relaxed2 X = relax2(K, Ss, rRc, rBc);
+    const int q1 = ready_wait();
+    const PlaneGrad2 gp = plane_grad2<WR>(sphi[q1], own);
+    const V2 H0 = v2(1.f / 3.f), H1 = v2(1.f / 12.f);  // W / 2
+    const V2 px = p_fma(H0, g0.gx, p_mul(H1, p_add(gm.gx, gp.gx)));
+    const V2 py = p_fma(H0, g0.gy, p_mul(H1, p_add(gm.gy, gp.gy)));
+    const V2 pz = p_mul(v2(0.5f), v_sub(gp.m, gm.m));
+    gm = g0;
+    g0 = gp;
+    const V2 psq = p_fma(px, px, p_fma(py, py, p_mul(pz, pz)));
+    const bool on0 = col0 && psq.x > 1.e-20f, on1 = col1 && psq.y > 1.e-20f;
+    auto store2 = [&](int l, V2 a, V2 b, bool s0, bool s1) {
+      S* const at = Bp.at(l, int(cell));
+      if (s0) SPair<S>::st(at, make_float2(a.x, b.x));
+      if (s1) SPair<S>::st(at + 32, make_float2(a.y, b.y));
+    };
+    if (on0 || on1)
+      recolour2<SD>(K, X, Ss, rRc, rBc, px, py, pz, psq, [&](int l, V2 a, V2 b) { store2(l, a, b, on0, on1); });
+    // cells without a colour gradient: the BGK result per component; solid
+    // cells: the plain pull
+    const bool off0 = col0 && !on0, off1 = col1 && !on1;
+    was_off = __any_sync(0xffffffffu, off0 || off1);
+    if (off0 || off1) {
+      R ra[Q], rb[Q];
+      if (keep) {
+#pragma unroll
+        for (int l = 0; l < Q; ++l) {
+          ra[l] = staged0(l);
+          rb[l] = staged1(l);
+        }
+      } else {
+#pragma unroll
+        for (int l = 0; l < Q; ++l) {
+          ra[l] = rb[l] = R{};
+          if (off0) ra[l] = SPair<S>::ldr(Ap.at(l, pull_one(g, x0 + c, y0 + ty, z, l)));
+          if (off1) rb[l] = SPair<S>::ldr(Ap.at(l, pull_one(g, x0 + 16 + c, y0 + ty, z, l)));
+        }
+      }
+      bgk2<SD>(
+          K, X, SD ? p_add(rRc, rBc) : rRc, SD ? v_sub(rRc, rBc) : rBc,
+          [&](int l, V2& a, V2& b) {
+            const V2 p0 = SPair<S>::cvt(ra[l]), p1 = SPair<S>::cvt(rb[l]);
+            a = make_float2(p0.x, p1.x);
+            b = make_float2(p0.y, p1.y);
+          },
+          [&](int l, V2 a, V2 b) { store2(l, a, b, off0, off1); });
+    }
+    if (keep) mbar_arrive(emptyb + qz);
+    qz = q1;
+  }
+  mbar_arrive(emptyb + qz);  // plane zend is read
+}
+
+// Registers of the two roles: a CTA is launched with 128 per thread; the phase
+// warps give back what they do not need and the collision warps take it
+// (56 + 200 = 2 x 128).
+__device__ __forceinline__ void phase_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 56;"); }
+__device__ __forceinline__ void collide_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 200;"); }
+
+template <typename S, int TY, bool PART, bool SD>
+__global__ void __launch_bounds__(32 * TY, TY == 8 ? 2 : 1)
+    k_cg_lean2(const S* __restrict__ A, S* __restrict__ B, Geom g, LeanConst<float> K, int zlen,
+               unsigned long long* err, int64_t step, LeanPart<float> PT, const int4* __restrict__ plan) {
+  extern __shared__ __align__(16) unsigned char lean_smem[];
+  using M = Col2<S, TY, PART>;
+  M::init(lean_smem);
+  __syncthreads();
+  // the column and z-segment of this CTA: from the grid (equal segments) or
+  // from the launch's plan (x0, y0, z0, zend per CTA)
+  int x0 = blockIdx.x * 32, y0 = blockIdx.y * TY, z0 = blockIdx.z * zlen, z1 = min(z0 + zlen, g.nz);
+  if (plan) {
+    const int4 w = plan[blockIdx.x];
+    x0 = w.x;
+    y0 = w.y;
+    z0 = w.z;
+    z1 = w.w;
+  }
+  if (threadIdx.x >= M::NT) {
+    phase_registers();
+    PhaseSync sy;
+    phase_column2<S, TY, PART, SD>(A, g, K, x0, y0, z0, z1, err, step, PT, lean_smem, sy);
+  } else {
+    collide_registers();
+    SlotSeq sy;
+    collide_column2<S, TY, PART, SD>(A, B, g, K, x0, y0, z0, z1, err, step, PART && PT.fnew != nullptr, lean_smem, sy);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Several independent boxes in one persistent launch: each CTA takes work
 // items (box, column, z-segment) from a table, longest first, and marches
 // them like k_cg_lean.  Used by the ensemble of uneven boxes.
@@ -1322,6 +1896,37 @@ __global__ void __launch_bounds__(TX* TY, MINB)
                                                 bd.err, bd.step, bd.pt, M::phi(lean_smem), M::stage(lean_smem),
                                                 M::side(lean_smem), M::bar(lean_smem), sy);
     __syncthreads();  // the window and the stage are reused by the next item
+  }
+}
+
+template <typename S, int TY, bool PART, bool SD>
+__global__ void __launch_bounds__(32 * TY, TY == 8 ? 2 : 1)
+    k_cg_lean2_multi(const BoxDesc<float>* __restrict__ boxes, const WorkItem* __restrict__ work, int nwork,
+                     LeanConst<float> K) {
+  extern __shared__ __align__(16) unsigned char lean_smem[];
+  using M = Col2<S, TY, PART>;
+  M::init(lean_smem);
+  __syncthreads();
+  // the roles go through the same items; the slot barriers alone order them,
+  // so the copies of an item start while the one before is still collided
+  if (threadIdx.x >= M::NT) {
+    phase_registers();
+    PhaseSync sy;
+    for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
+      const WorkItem it = work[w];
+      const BoxDesc<float> bd = boxes[it.box];
+      phase_column2<S, TY, PART, SD>((const S*)bd.A, bd.g, K, it.x0, it.y0, it.z0, it.zend, bd.err, bd.step,
+                                            bd.pt, lean_smem, sy);
+    }
+  } else {
+    collide_registers();
+    SlotSeq sy;
+    for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
+      const WorkItem it = work[w];
+      const BoxDesc<float> bd = boxes[it.box];
+      collide_column2<S, TY, PART, SD>((const S*)bd.A, (S*)bd.B, bd.g, K, it.x0, it.y0, it.z0, it.zend, bd.err,
+                                              bd.step, PART && bd.pt.fnew != nullptr, lean_smem, sy);
+    }
   }
 }
 
@@ -1473,6 +2078,12 @@ static int prepare_lean_multi() {
                     done);
 }
 
+template <typename S, int TY, bool SD>
+static int prepare_lean2_multi() {
+  static unsigned long long done = 0;
+  return allow_smem(k_cg_lean2_multi<S, TY, true, SD>, Col2<S, TY, true>::BYTES, done);
+}
+
 // Box copies (16-bit storage): when nx is a multiple of 4 (a 16-byte granule
 // then never straddles the periodic x edge) unless switched off
 static bool use_boxes(const Ctx& c, bool part = false) {
@@ -1506,10 +2117,54 @@ static int launch_lean_as(Ctx& c, int zlen_override, LeanPart<typename Store<S>:
   return 0;
 }
 
+template <typename S, int TY, bool SD>
+static int launch_lean2(Ctx& c, int zlen_override) {
+  using M = Col2<S, TY, false>;
+  static unsigned long long done = 0;
+  static int per_sm[64] = {0}, sms[64] = {0};
+  auto* kernel = k_cg_lean2<S, TY, false, SD>;
+  int rc = allow_smem(kernel, M::BYTES, done);
+  if (rc) return rc;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return LBX_ERR_CUDA;
+  dev &= 63;
+  if (!per_sm[dev]) {
+    int nb = 0, nsm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, 2 * M::NT, M::BYTES) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nb < 1 || nsm < 1)
+      return LBX_ERR_CUDA;
+    sms[dev] = nsm;
+    per_sm[dev] = nb;
+  }
+  const int resident = per_sm[dev] * sms[dev];
+  const int zlen = zlen_override > 0 ? zlen_override : lean_zlen(c, 32, TY, resident);
+  dim3 grid((c.nx + 31) / 32, (c.ny + TY - 1) / TY, (c.nz + zlen - 1) / zlen);
+  int nplan = 0;
+  const int4* plan = nullptr;
+  if (zlen_override <= 0) plan = paired_plan(c, 32, TY, resident, &nplan);
+  if (!plan && c.zhi > 0) {  // a z-slab: only its own planes
+    plan = range_plan(c, 32, TY, resident, &nplan);
+    if (!plan) return LBX_ERR_ALLOC;
+  }
+  if (plan) grid = dim3(unsigned(nplan), 1, 1);
+  kernel<<<grid, 2 * M::NT, M::BYTES, c.stream>>>((const S*)c.pops[c.cur], (S*)c.pops[1 - c.cur], geom(c),
+                                              make_lean<float>(c), zlen, c.d_err, c.step + 1, LeanPart<float>{}, plan);
+  return 0;
+}
+
 template <typename S, int TX, int TY, int MINB, bool PART, bool SD = false, bool SDP = false>
 static int launch_lean(Ctx& c, int zlen_override, LeanPart<typename Store<S>::C> pt) {
   if constexpr (kStaged<S, PART>) {
-    if (use_boxes(c, PART)) return launch_lean_as<S, TX, TY, MINB, PART, SD, SDP, true>(c, zlen_override, pt);
+    // Two cells per thread in two roles, except where that is slower: with
+    // spheres (721 us of the colloid step against 695 at 256^3 with 1280
+    // spheres: flags and solid cells lengthen both roles) and with the
+    // predicted split (86.6 against 84.3 us at FP16 128^3: a window read per
+    // direction in the collision's chain)
+    if constexpr (PART || SDP) {
+      if (use_boxes(c, PART)) return launch_lean_as<S, TX, TY, MINB, PART, SD, SDP, true>(c, zlen_override, pt);
+    } else {
+      if (use_boxes(c)) return launch_lean2<S, TY, SD>(c, zlen_override);
+    }
   }
   return launch_lean_as<S, TX, TY, MINB, PART, SD, SDP, false>(c, zlen_override, pt);
 }
@@ -1577,10 +2232,11 @@ int ensemble_launch(const std::vector<Ctx*>& boxes, int shape, const std::vector
   if (boxes.empty()) return LBX_ERR_ARG;
   const Ctx& c0 = *boxes[0];
   const int TX = 32, TY = shape == 1 ? 16 : 8;
-  // The persistent kernel keeps each work item's box descriptor in
-  // registers, which leaves no room for the box copies' per-thread state
-  // without spills (measured: 8-16 bytes per thread), so it stages its 16-bit
-  // pulls one copy per pull (BOX = false).
+  // 16-bit storage on widths that are multiples of 4 (every box with spheres
+  // is): the kernel with two cells per thread; otherwise one copy per pull
+  // (the one-cell kernel's box copies would spill beside an item's descriptor)
+  bool wide = true;
+  for (const Ctx* c : boxes) wide = wide && c->nx % 4 == 0;
   return by_storage(c0, [&](auto* tag) -> int {
     using S = std::remove_pointer_t<decltype(tag)>;
     using C = typename Store<S>::C;
@@ -1615,11 +2271,11 @@ int ensemble_launch(const std::vector<Ctx*>& boxes, int shape, const std::vector
         rp = prepare_lean_multi<S, 32, 16, 1, true>();
         if (!rp) rp = prepare_lean_multi<S, 32, 8, 2, true>();
       } else if (c0.sd) {
-        rp = prepare_lean_multi<S, 32, 16, 1, true, true>();
-        if (!rp) rp = prepare_lean_multi<S, 32, 8, 2, true, true>();
+        rp = wide ? prepare_lean2_multi<S, 16, true>() : prepare_lean_multi<S, 32, 16, 1, true, true>();
+        if (!rp) rp = wide ? prepare_lean2_multi<S, 8, true>() : prepare_lean_multi<S, 32, 8, 2, true, true>();
       } else {
-        rp = prepare_lean_multi<S, 32, 16, 1, true>();
-        if (!rp) rp = prepare_lean_multi<S, 32, 8, 2, true>();
+        rp = wide ? prepare_lean2_multi<S, 16, false>() : prepare_lean_multi<S, 32, 16, 1, true>();
+        if (!rp) rp = wide ? prepare_lean2_multi<S, 8, false>() : prepare_lean_multi<S, 32, 8, 2, true>();
       }
       if (rp) return rp;
       if (cudaMemcpy(d_desc, desc.data(), desc.size() * sizeof(BoxDesc<C>), cudaMemcpyHostToDevice) != cudaSuccess)
@@ -1644,7 +2300,14 @@ int ensemble_launch(const std::vector<Ctx*>& boxes, int shape, const std::vector
     } else {
       auto go = [&](auto sd_tag) {
         constexpr bool SDV = decltype(sd_tag)::value;
-        if (shape == 1)
+        using W16 = Col2<S, 16, true>;
+        using W8 = Col2<S, 8, true>;
+        if (wide && shape == 1)
+          k_cg_lean2_multi<S, 16, true, SDV>
+              <<<std::min(nwork, 148), 2 * W16::NT, W16::BYTES, stream>>>(D, W, nwork, K);
+        else if (wide)
+          k_cg_lean2_multi<S, 8, true, SDV><<<std::min(nwork, 296), 2 * W8::NT, W8::BYTES, stream>>>(D, W, nwork, K);
+        else if (shape == 1)
           k_cg_lean_multi<S, 32, 16, 1, true, SDV>
               <<<std::min(nwork, 148), dim3(32, 16), LeanSmem<S, 32, 16, true>::BYTES, stream>>>(D, W, nwork, K);
         else

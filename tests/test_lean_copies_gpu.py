@@ -75,3 +75,28 @@ def test_moving_spheres_copies_bit_identical(storage, n):
         assert np.array_equal(a, b)
     for k in ra:
         assert np.array_equal(ra[k], rb[k]), k
+
+
+def _half_plain_run(storage, copies, cta, plain, nx=72, ny=20, nz=24, steps=6):
+    """A box whose cells with x < plain hold one fluid at rest density (no colour gradient there)."""
+    rR, rB = seeded_noise_fields(nx, ny, nz, seed=9)
+    rR[:, :, :plain] = 1.0
+    rB[:, :, :plain] = 0.0
+    g = LBSim(make_params(nx, ny, nz, model="cg", storage=storage, sigma=0.02, beta=0.7))
+    g.set_lean_copies(copies)
+    g.set_lean_shape(cta, 0)
+    g.set_fields(rR, rB)
+    g.step(steps)
+    out = g.get_pops()
+    g.close()
+    return out
+
+
+@pytest.mark.parametrize("storage", ["f16", "bf16", "f16sd"])
+@pytest.mark.parametrize("cta,plain", [(0, 72), (0, 40), (0, 21), (1, 40)])
+def test_cells_without_a_gradient(storage, cta, plain):
+    """The two-cell kernel gives a cell without a colour gradient its pairs a second time, from the stage or from
+    L2, with both, one or none of a thread's cells in the bulk of one fluid: the same bits as the per-pull kernel."""
+    a, b = (_half_plain_run(storage, m, cta, plain) for m in (1, 0))
+    for p, q in zip(a, b):
+        assert np.isfinite(p).all() and np.array_equal(p, q)
