@@ -39,10 +39,10 @@ extern "C" {
 #define LBX_MODEL_BGK 0 /* single-component BGK (kernels_fluid_BGK.CUF)        */
 #define LBX_MODEL_CG 1  /* two-component colour gradient (kernels_fluid_CG.CUF) */
 #define LBX_MODEL_CG_DIFFDENS 2 /* colour gradient with two fluid densities (the DIFFDENS build,
-                                 kernels_fluid_CG.CUF:40-49,163-177,539-819): two-pass schedule */
+                                 kernels_fluid_CG.CUF:40-49,163-177,539-819): schedule 0 */
 #define LBX_MODEL_CG_D3Q27 3    /* colour gradient on the D3Q27 lattice (the D3Q27 build,
                                    dimensions_m.CUF:117-198): 27 populations per component,
-                                   two-pass schedule, no spheres (the reference's bounce-back is
+                                   schedule 0, no spheres (the reference's bounce-back is
                                    D3Q19 only, kernels_fluid_PART.CUF:1929-1941) */
 #define LBX_MODEL_CG_DIFFDENS_D3Q27 4 /* both builds together */
 
@@ -334,7 +334,8 @@ int lbx_get_stream(void* ctx, void** stream);
 /* ---- measurement ------------------------------------------------------- */
 /* Colour-gradient schedule: 2 = lean single-pass kernel (default), 1 = the
  * first single-pass kernel, 0 = two passes (phase field, then collision).
- * LBX_MODEL_CG_DIFFDENS runs on 0 only (other values: LBX_ERR_ARG).
+ * The two-density and D3Q27 models take 0 only (other values: LBX_ERR_ARG);
+ * without spheres lbx_step fuses its two passes into one, bit for bit equal.
  * The reference prints Mlup/s from CUDA events around the step loop
  * (main.CUF:274-292); these are the hooks the benchmark uses for the same. */
 int lbx_set_schedule(void* ctx, int32_t fused);
