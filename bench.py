@@ -335,12 +335,12 @@ def colloid_timing(storage, steps=50, warm=10, small=False):
 
 def variants_timing(storage, steps=100, warm=20):
     """The reference's compile-time variants as models (densR = 2, densB = 1 for the two-density ones,
-    as in its namelist deck): the spinodal workload at 128^3 on the two-pass schedule (phase field /
-    densities, then the collision), single density on D3Q19 beside them for scale."""
+    as in its namelist deck): the spinodal workload at 128^3, one pass per step; the single density on D3Q19
+    in two passes (phase field, then the collision) beside them for scale."""
     from lbcuda_b200 import LBSim, make_params
     from lbcuda_b200.inputs import seeded_noise_fields
     rR, rB = seeded_noise_fields(L, L, L, seed=SEED)
-    out = {"storage": storage, "densR": 2.0, "densB": 1.0, "schedule": "two-pass"}
+    out = {"storage": storage, "densR": 2.0, "densB": 1.0, "schedule": "0 (cg: two passes; the other models: one)"}
     for model in ("cg", "cg-diffdens", "cg-d3q27", "cg-diffdens-d3q27"):
         s = LBSim(make_params(L, model=model, storage=storage, sigma=SIGMA, beta=BETA, densR=2.0, densB=1.0))
         s.set_schedule(0)
