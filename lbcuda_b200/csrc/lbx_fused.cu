@@ -35,6 +35,7 @@
 // cells per thread and two roles per CTA (phase_column2 and
 // collide_column2 below); the results are the same bits.
 #include "lbx_device.cuh"
+#include "lbx_roles.h"
 
 #include <algorithm>
 #include <type_traits>
@@ -1825,11 +1826,14 @@ __device__ __forceinline__ void collide_column2(const S* __restrict__ A, S* __re
   mbar_arrive(emptyb + qz);  // plane zend is read
 }
 
-// Registers of the two roles: a CTA is launched with 128 per thread; the phase
-// warps give back what they do not need and the collision warps take it
-// (56 + 200 = 2 x 128).
-__device__ __forceinline__ void phase_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 56;"); }
-__device__ __forceinline__ void collide_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 200;"); }
+// Registers of the two roles (lbx_roles.h): the phase warps give back what they
+// do not need and the collision warps take it.
+__device__ __forceinline__ void phase_registers() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPhaseRegs));
+}
+__device__ __forceinline__ void collide_registers() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kCollideRegs));
+}
 
 template <typename S, int TY, bool PART, bool SD>
 __global__ void __launch_bounds__(32 * TY, TY == 8 ? 2 : 1)
@@ -2078,6 +2082,20 @@ static int prepare_lean_multi() {
                     done);
 }
 
+// Whether this build launches a two-role kernel with the registers its roles
+// share out (they would wait for the missing ones without a limit); where not,
+// the caller takes the one-copy-per-pull kernel, which gives the same bits.
+template <typename K>
+static bool roles_fit(K* kernel) {
+  cudaFuncAttributes at;
+  return cudaFuncGetAttributes(&at, kernel) == cudaSuccess && role_regs_fit(at.numRegs);
+}
+template <typename S, bool SD>
+static bool multi_roles_fit() {
+  static const bool fit = roles_fit(k_cg_lean2_multi<S, 8, true, SD>) && roles_fit(k_cg_lean2_multi<S, 16, true, SD>);
+  return fit;
+}
+
 template <typename S, int TY, bool SD>
 static int prepare_lean2_multi() {
   static unsigned long long done = 0;
@@ -2163,7 +2181,8 @@ static int launch_lean(Ctx& c, int zlen_override, LeanPart<typename Store<S>::C>
     if constexpr (PART || SDP) {
       if (use_boxes(c, PART)) return launch_lean_as<S, TX, TY, MINB, PART, SD, SDP, true>(c, zlen_override, pt);
     } else {
-      if (use_boxes(c)) return launch_lean2<S, TY, SD>(c, zlen_override);
+      static const bool fit = roles_fit(k_cg_lean2<S, TY, false, SD>);
+      if (fit && use_boxes(c)) return launch_lean2<S, TY, SD>(c, zlen_override);
     }
   }
   return launch_lean_as<S, TX, TY, MINB, PART, SD, SDP, false>(c, zlen_override, pt);
@@ -2240,6 +2259,7 @@ int ensemble_launch(const std::vector<Ctx*>& boxes, int shape, const std::vector
   return by_storage(c0, [&](auto* tag) -> int {
     using S = std::remove_pointer_t<decltype(tag)>;
     using C = typename Store<S>::C;
+    if constexpr (sizeof(S) == 2) wide = wide && (c0.sd ? multi_roles_fit<S, true>() : multi_roles_fit<S, false>());
     if (build_only) {
       std::vector<BoxDesc<C>> desc(boxes.size());
       std::vector<WorkItem> work;

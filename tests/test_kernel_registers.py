@@ -18,17 +18,26 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 
 
-def test_lean_kernels_do_not_spill(tmp_path):
+def _ptxas_report(source):
+    """Lines of the ptxas statistics of one source file, compiled as the build compiles it."""
     from lbcuda_b200 import build as B
     nvcc = B.nvcc()
     if not (os.path.isabs(nvcc) and os.path.exists(nvcc)) and shutil.which(nvcc) is None:
         pytest.skip("nvcc not available")
-    src = os.path.join(B.CSRC, "lbx_fused.cu")
-    cmd = [nvcc] + B.NVCC_FLAGS + B.FILE_FLAGS.get("lbx_fused.cu", []) + ["-Xptxas", "-v", "-c", src, "-o",
-                                                                          str(tmp_path / "f.o")]
+    cmd = [nvcc] + B.NVCC_FLAGS + B.FILE_FLAGS.get(source, []) + ["-Xptxas", "-v", "-c", os.path.join(B.CSRC, source),
+                                                                  "-o", os.devnull]
     p = subprocess.run(cmd, capture_output=True, text=True)
     assert p.returncode == 0, p.stderr[-2000:]
-    lines = p.stderr.splitlines()
+    return p.stderr.splitlines()
+
+
+@pytest.fixture(scope="module")
+def fused_report():
+    return _ptxas_report("lbx_fused.cu")
+
+
+def test_lean_kernels_do_not_spill(fused_report):
+    lines = fused_report
     cur = None
     checked = 0
     bad = []
@@ -46,3 +55,30 @@ def test_lean_kernels_do_not_spill(tmp_path):
                 bad.append((cur, m.group(1), m.group(2)))
     assert checked >= 8, "no k_cg_lean instantiations found in the ptxas output"
     assert not bad, f"register spills in single-pass kernels: {bad}"
+
+
+def test_two_role_kernels_launch_with_the_registers_they_share_out(fused_report):
+    """k_cg_lean2 hands registers from its phase warps to its collision warps (setmaxnreg), which wait without a
+    limit for any the launch did not allocate; every instance of this build is launched with the number that the
+    two shares are made for."""
+    cur, used = None, {}
+    for line in fused_report:
+        m = re.search(r"Compiling entry function '(\S+)'", line)
+        cur = m.group(1) if m else cur
+        m = re.search(r"Used (\d+) registers", line)
+        if m and cur and "k_cg_lean2" in cur:
+            used[cur] = int(m.group(1))
+    assert len(used) >= 12 and set(used.values()) == {128}, used
+
+
+def test_role_shares_are_checked_against_the_launch(tmp_path):
+    """The host takes the two-role kernels only where the launch allocation holds both shares (56 + 200 for two
+    threads): not with one register less, and not with a share on the wrong side of the allocation."""
+    from lbcuda_b200 import build as B
+    src = tmp_path / "roles.cpp"
+    src.write_text('#include "lbx_roles.h"\n#include <cstdio>\n'
+                   'int main() { for (int r = 24; r <= 255; ++r) if (lbx::role_regs_fit(r)) std::printf("%d\\n", r); }\n')
+    exe = str(tmp_path / "roles")
+    subprocess.run(["g++", "-std=c++17", "-I", B.CSRC, str(src), "-o", exe], check=True)
+    fits = [int(v) for v in subprocess.run([exe], capture_output=True, text=True, check=True).stdout.split()]
+    assert fits == list(range(128, 201))
