@@ -326,21 +326,19 @@ __global__ void __launch_bounds__(TX* TY) k_cg_fused(const S* __restrict__ A, S*
 
 // ---------------------------------------------------------------------------
 // Single-pass step of the models that keep the reference's per-component
-// collision: two fluid densities (DD) and the D3Q27 lattice.  A CTA marches
-// the column [x0, x0+32) x [y0, y0+8) along z over one segment.  Per plane it
-// sums the pulls of plane z+1 for its cells and the ring around them into
-// densities and writes their phase field (DD: and the densities) into a
-// four-plane shared window, then pulls plane z again (from L1 / L2, where the
-// sums left it), takes the gradients from the window, collides and stores.
-// The helpers and their order are those of k_cg_phi and k_cg_collide, so the
-// results are theirs bit for bit.
-// Bound: HBM, which the two passes read twice for the populations and once
-// more for the phase field and the densities.  Two densities at 128^3 FP32:
-// 187 us per step against 244 in two passes (304 bytes per cell: 99 us at the
-// copy rate); D3Q27 at 96^3 FP32: 123 us against 151 (432 bytes: 59 us).
+// collision: two fluid densities (DD) and the D3Q27 lattice.  A CTA marches a
+// column of w x h cells along z over one segment.  Per plane it sums the pulls
+// of plane z+1 for its cells and the ring around them into densities and writes
+// their phase field (DD: and the densities) into a four-plane shared window,
+// then pulls plane z again (from L1 / L2, where the sums left it), takes the
+// gradients from the window, collides and stores.  The helpers and their order
+// are those of k_cg_phi and k_cg_collide, so the results are theirs bit for bit.
+// Bound: the chain of a plane (pull, sum, barrier, pull, collide): 5.0 us for a
+// CTA alone on its SM, 6.4 us with two, at FP32 with two densities, whatever
+// the cells do.  So the time follows the planes per resident CTA, and the
+// column's shape and the segments decide (march_plan); columns of 32 x 8 on
+// every box took 43 us a step at 65 x 57 x 49, 22 of 24 columns being partial.
 // ---------------------------------------------------------------------------
-constexpr int MTX = 32, MTY = 8;
-
 template <typename S> struct Pair2;  // the two components of a direction and cell as one word
 template <> struct Pair2<float> { using R = float2; };
 template <> struct Pair2<double> { using R = double2; };
@@ -360,39 +358,48 @@ __device__ __forceinline__ void pull_pairs(const S* __restrict__ A, const Geom& 
   }
 }
 
-__device__ __forceinline__ int wrap_into(int v, int n) {
-  v %= n;
-  return v < 0 ? v + n : v;
-}
-
 template <typename S, bool DD, int QQ>
-__global__ void __launch_bounds__(MTX* MTY, sizeof(typename Store<S>::C) == 4 ? 2 : 1)
+__global__ void __launch_bounds__(March<typename Store<S>::C>::NT, sizeof(typename Store<S>::C) == 4 ? 2 : 1)
     k_cg_march(const S* __restrict__ A, S* __restrict__ B, Geom g, Shift<typename Store<S>::C> sh,
-               CGConst<typename Store<S>::C> K, int zlen, unsigned long long* err, int64_t step) {
+               CGConst<typename Store<S>::C> K, MarchPlan P, unsigned long long* err, int64_t step) {
   using C = typename Store<S>::C;
   using R = typename Pair2<S>::R;
-  constexpr int RX = MTX + 2, CELLS = RX * (MTY + 2), NRING = 2 * RX + 2 * MTY;
+  using M = March<C>;
+  constexpr int RX = M::PITCH, CELLS = M::PITCH * M::ROWS;
   __shared__ C win[4][DD ? 3 : 1][CELLS];  // phase field, densities
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * MTX + tx;
-  const int x0 = blockIdx.x * MTX, y0 = blockIdx.y * MTY, z0 = blockIdx.z * zlen, zend = min(z0 + zlen, g.nz);
-  // a partial column still fills its window (wrapped positions); only cells
-  // of the box collide
-  const bool active = x0 + tx < g.nx && y0 + ty < g.ny;
-  const int x = wrap_into(x0 + tx, g.nx), y = wrap_into(y0 + ty, g.ny);
+  const int tid = threadIdx.x;
+  const int seg = blockIdx.x / P.cols, col = blockIdx.x - seg * P.cols, cy = col / P.kx, cx = col - cy * P.kx;
+  const int x0 = cx * P.w, y0 = cy * P.h, z0 = seg * P.zlen, zend = min(z0 + P.zlen, g.nz);
+  const int w = min(P.w, g.nx - x0), h = min(P.h, g.ny - y0);  // a column at the box's end is cut to it
+  // the first w h threads own a cell each, the last ones a cell of the ring
+  const int ty = tid / w, tx = tid - ty * w;
+  const bool active = ty < h;
+  const int x = x0 + tx, y = y0 + ty;
   const int own = (ty + 1) * RX + tx + 1;
-  // ring cell of this thread (threads 0 .. NRING-1)
+  const int rid = M::NT - 1 - tid;
+  const bool ringer = rid < 2 * (w + 2) + 2 * h;
   int rx = 0, ry = 0;
-  if (tid < RX) { rx = tid; }
-  else if (tid < 2 * RX) { rx = tid - RX; ry = MTY + 1; }
-  else if (tid < 2 * RX + MTY) { ry = 1 + tid - 2 * RX; }
-  else if (tid < NRING) { rx = RX - 1; ry = 1 + tid - 2 * RX - MTY; }
-  const bool ringer = tid < NRING;
-  const int rxg = wrap_into(x0 + rx - 1, g.nx), ryg = wrap_into(y0 + ry - 1, g.ny), rslot = ry * RX + rx;
+  if (rid < w + 2) { rx = rid; }
+  else if (rid < 2 * (w + 2)) { rx = rid - (w + 2); ry = h + 1; }
+  else if (rid < 2 * (w + 2) + h) { ry = 1 + rid - 2 * (w + 2); }
+  else { rx = w + 1; ry = 1 + rid - 2 * (w + 2) - h; }
+  const int rxg = wrapc(x0 + rx - 1, g.nx), ryg = wrapc(y0 + ry - 1, g.ny), rslot = ry * RX + rx;
+  // its place waits in shared memory: held in registers it spills 8 to 20 bytes
+  // (104 against 96 us at 96^3, FP16, two densities); FP64, with 255 registers,
+  // spills the other way round
+  constexpr bool PARK = sizeof(C) == 4;
+  __shared__ int ring[PARK ? M::RING : 1][3];
+  if constexpr (PARK)
+    if (ringer) {
+      ring[rid][0] = rxg;
+      ring[rid][1] = ryg;
+      ring[rid][2] = rslot;
+    }
 
-  // densities and phase field of cell (cx, cy) of plane p into its window slot
-  auto fill = [&](int cx, int cy, int p, int slot, bool check) {
+  // densities and phase field of cell (px, py) of plane p into its window slot
+  auto fill = [&](int px, int py, int p, int slot, bool check) {
     Nbr b;
-    make_nbr(g, cx, cy, wrap_into(p, g.nz), b);
+    make_nbr(g, px, py, wrapc(p, g.nz), b);
     C fR[QQ], fB[QQ];
     pull_pairs<QQ>(A, g, b, sh, fR, fB);
     C rR = sum_q<QQ>(fR), rB = sum_q<QQ>(fB);
@@ -407,8 +414,11 @@ __global__ void __launch_bounds__(MTX* MTY, sizeof(typename Store<S>::C) == 4 ? 
     }
   };
   auto plane = [&](int p) {
-    fill(x, y, p, own, active && p >= z0 && p < zend);
-    if (ringer) fill(rxg, ryg, p, rslot, false);
+    if (active) fill(x, y, p, own, p >= z0 && p < zend);
+    if (ringer) {
+      if constexpr (PARK) fill(ring[rid][0], ring[rid][1], p, ring[rid][2], false);
+      else fill(rxg, ryg, p, rslot, false);
+    }
   };
   plane(z0 - 1);
   plane(z0);
@@ -784,48 +794,35 @@ int fluid_fused(Ctx& c) {
   });
 }
 
-// Segments of k_cg_march: the count that makes waves of resident CTAs times
-// planes per segment (with its two extra planes) smallest, the fewest of equal
-// ones, since long segments keep neighbouring columns in step.
-static int march_zlen(const Ctx& c) {
-  const long cols = long((c.nx + MTX - 1) / MTX) * long((c.ny + MTY - 1) / MTY);
-  const long resident = 148L * (c.storage == LBX_STORE_F64 ? 1 : 2);
-  long best = 0;
-  int zlen = c.nz;
-  for (int segs = 1; segs <= c.nz; ++segs) {
-    const int len = (c.nz + segs - 1) / segs;
-    const long n = cols * ((c.nz + len - 1) / len), cost = ((n + resident - 1) / resident) * (len + 2);
-    if (!best || cost < best) {
-      best = cost;
-      zlen = len;
-    }
+template <typename S, bool DD, int QQ>
+static int launch_march(Ctx& c) {
+  using C = typename Store<S>::C;
+  auto* kernel = k_cg_march<S, DD, QQ>;
+  if (!c.march.w) {  // this box's plan, once
+    int dev = 0, sms = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, March<C>::NT, 0) != cudaSuccess || per_sm < 1)
+      return LBX_ERR_CUDA;
+    c.march = march_plan<C>(c.nx, c.ny, c.nz, sms * per_sm, sizeof(S) == 4);
   }
-  return zlen;
+  MarchPlan P = c.march;
+  if (c.lean_zlen > 0) P.zlen = std::min(c.lean_zlen, c.nz);
+  kt_begin(c);
+  kernel<<<P.cols * ((c.nz + P.zlen - 1) / P.zlen), March<C>::NT, 0, c.stream>>>(
+      (const S*)c.pops[c.cur], (S*)c.pops[1 - c.cur], geom(c), make_shift<C>(c), make_cg<C>(c), P, c.d_err, c.step + 1);
+  kt_end(c);
+  c.cur = 1 - c.cur;
+  return launch_status();
 }
 
 static int fluid_march(Ctx& c) {
-  const int zlen = march_zlen(c);
-  const dim3 block(MTX, MTY, 1);
-  const dim3 grid((c.nx + MTX - 1) / MTX, (c.ny + MTY - 1) / MTY, (c.nz + zlen - 1) / zlen);
   return by_storage(c, [&](auto* tag) {
     using S = std::remove_pointer_t<decltype(tag)>;
-    using C = typename Store<S>::C;
-    kt_begin(c);
-    const S* A = (const S*)c.pops[c.cur];
-    S* B = (S*)c.pops[1 - c.cur];
     const bool dd = two_densities(c);
-    if (dd && c.q == Q27)
-      k_cg_march<S, true, Q27><<<grid, block, 0, c.stream>>>(A, B, geom(c), make_shift<C>(c), make_cg<C>(c), zlen,
-                                                            c.d_err, c.step + 1);
-    else if (dd)
-      k_cg_march<S, true, Q><<<grid, block, 0, c.stream>>>(A, B, geom(c), make_shift<C>(c), make_cg<C>(c), zlen,
-                                                          c.d_err, c.step + 1);
-    else
-      k_cg_march<S, false, Q27><<<grid, block, 0, c.stream>>>(A, B, geom(c), make_shift<C>(c), make_cg<C>(c), zlen,
-                                                             c.d_err, c.step + 1);
-    kt_end(c);
-    c.cur = 1 - c.cur;
-    return launch_status();
+    if (dd && c.q == Q27) return launch_march<S, true, Q27>(c);
+    if (dd) return launch_march<S, true, Q>(c);
+    return launch_march<S, false, Q27>(c);
   });
 }
 
