@@ -842,6 +842,24 @@ int fluid_bgk(Ctx& c) {
   });
 }
 
+// Whether a step of the two-density and D3Q27 models takes k_cg_march.  FP32 and
+// FP64 pairs, both models at once, and FP16 with two densities: always (1.3 times
+// as fast as two passes on average; down to 0.91 in the first steps of a droplet,
+// FP64 with 56^3 cells, and 0.97 to 0.98 in FP32 around 44^3 to 64^3).  The other
+// 16-bit models: not between small boxes, where it saves a launch, and a million
+// cells.  There the two passes gain more from the cells of one fluid, which they
+// do not recolour, and a box of two fluids is mostly such cells once it has
+// separated.  Two passes against one, us per step on a droplet [on noise]:
+//   D3Q27 FP16      40^3 21.3, 18.8 [24.7, 20.1]   64^3 37.2, 40.2 [45.2, 39.6]
+//                   88^3 90.7, 96.2 [116, 98]     100^3  149,  127 [194, 137]
+//   2 densities     40^3 20.6, 17.8 [23.7, 18.6]   64^3 33.5, 37.9 [39.2, 35.4]
+//   BF16            88^3 81.5, 87.6 [97.7, 84.2]  100^3  141,  119 [174, 115]
+static bool single_pass(const Ctx& c) {
+  const bool both = two_densities(c) && c.q == Q27;
+  if (c.elem != 2 || both || (two_densities(c) && c.storage == LBX_STORE_F16)) return true;
+  return c.n <= 64000 || c.n >= 1000000;
+}
+
 int fluid_step(Ctx& c) {
   int rc;
   if (c.ncomp == 1) {
@@ -850,7 +868,7 @@ int fluid_step(Ctx& c) {
     rc = fluid_lean(c);
   } else if (c.fused == 1) {
     rc = fluid_fused(c);
-  } else if (c.p.model != LBX_MODEL_CG) {  // two densities, D3Q27
+  } else if (c.p.model != LBX_MODEL_CG && single_pass(c)) {
     rc = fluid_march(c);
   } else {
     rc = fluid_init_rho(c);

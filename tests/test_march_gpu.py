@@ -55,3 +55,23 @@ def test_window_reused_over_long_segments(model, storage, shape, zlen):
     assert a.status()[0] == 0
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("model,storage", [("cg-diffdens", "bf16"), ("cg-d3q27", "f16"), ("cg-d3q27", "bf16"),
+                                           ("cg-diffdens", "f16")])
+@pytest.mark.parametrize("nx", [40, 41])
+def test_both_sides_of_the_small_box_rule(model, storage, nx):
+    """64,000 cells and a few more: some 16-bit models go back to two passes there; the step is the same."""
+    rR, rB = seeded_noise_fields(nx, 40, 40, seed=8, amp=0.05)
+    a, b = (LBSim(make_params(nx, 40, 40, model=model, storage=storage, sigma=0.02, beta=0.7, densR=2.0, densB=1.0))
+            for _ in range(2))
+    for s in (a, b):
+        s.set_fields(rR, rB)
+    a.step(3)
+    for _ in range(3):
+        assert b._L.lbx_init_rho(b._h) == 0 and b._L.lbx_time_step_cg(b._h) == 0
+    for p, q in zip(a.get_pops(), b.get_pops()):
+        assert np.isfinite(p).all() and np.array_equal(p, q)
+    assert a.status()[0] == 0 and a.steps_taken == 3
+    a.close()
+    b.close()
