@@ -2135,7 +2135,7 @@ static int launch_lean_as(Ctx& c, int zlen_override, LeanPart<typename Store<S>:
   return 0;
 }
 
-template <typename S, int TY, bool SD>
+template <typename S, int TY, int MINB, bool SD>
 static int launch_lean2(Ctx& c, int zlen_override) {
   using M = Col2<S, TY, false>;
   static unsigned long long done = 0;
@@ -2156,6 +2156,14 @@ static int launch_lean2(Ctx& c, int zlen_override) {
   }
   const int resident = per_sm[dev] * sms[dev];
   const int zlen = zlen_override > 0 ? zlen_override : lean_zlen(c, 32, TY, resident);
+  // Component pairs in segments of one or two planes (boxes up to about 48^3):
+  // one copy per pull, since there is nothing for the second role to overlap and
+  // a cell without a gradient costs it more.  Two roles against one copy per
+  // pull, us per step, FP16, one fluid after 200 steps: 20^3 8.4, 6.3; 32^3 8.4,
+  // 7.5; 48^3 14.5, 12.5; 64^3 (four planes) 18.6, 18.6, noise 16.6, 17.7.  Not
+  // narrow boxes, whose copies start on few lines: 4 x 64 x 64 15.5, 16.5.
+  if (!SD && zlen <= 2 && zlen_override <= 0 && c.nx >= 12)
+    return launch_lean_as<S, 32, TY, MINB, false, SD, false, false>(c, zlen_override, LeanPart<float>{});
   dim3 grid((c.nx + 31) / 32, (c.ny + TY - 1) / TY, (c.nz + zlen - 1) / zlen);
   int nplan = 0;
   const int4* plan = nullptr;
@@ -2182,7 +2190,7 @@ static int launch_lean(Ctx& c, int zlen_override, LeanPart<typename Store<S>::C>
       if (use_boxes(c, PART)) return launch_lean_as<S, TX, TY, MINB, PART, SD, SDP, true>(c, zlen_override, pt);
     } else {
       static const bool fit = roles_fit(k_cg_lean2<S, TY, false, SD>);
-      if (fit && use_boxes(c)) return launch_lean2<S, TY, SD>(c, zlen_override);
+      if (fit && use_boxes(c)) return launch_lean2<S, TY, MINB, SD>(c, zlen_override);
     }
   }
   return launch_lean_as<S, TX, TY, MINB, PART, SD, SDP, false>(c, zlen_override, pt);

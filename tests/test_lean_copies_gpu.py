@@ -100,3 +100,14 @@ def test_cells_without_a_gradient(storage, cta, plain):
     a, b = (_half_plain_run(storage, m, cta, plain) for m in (1, 0))
     for p, q in zip(a, b):
         assert np.isfinite(p).all() and np.array_equal(p, q)
+
+
+@pytest.mark.parametrize("storage", ["f16", "bf16", "f16sd"])
+@pytest.mark.parametrize("shape", [(12, 12, 12), (8, 12, 12), (48, 48, 48), (52, 52, 52)])
+def test_small_boxes_take_either_kernel(storage, shape):
+    """The automatic segments on both sides of the rules for component pairs: one-plane segments 12 and 8 cells wide,
+    two planes (48^3) and three (52^3)."""
+    (pa, fa, sa), (pb, fb, sb) = (_fluid_run(shape, storage, m, 0, 0, 4) for m in (1, 0))
+    assert sa == 0 and sb == 0
+    for a, b in zip(pa + fa, pb + fb):
+        assert np.array_equal(a, b)
