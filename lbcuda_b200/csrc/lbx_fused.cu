@@ -2260,10 +2260,23 @@ int ensemble_launch(const std::vector<Ctx*>& boxes, int shape, const std::vector
   const Ctx& c0 = *boxes[0];
   const int TX = 32, TY = shape == 1 ? 16 : 8;
   // 16-bit storage on widths that are multiples of 4 (every box with spheres
-  // is): the kernel with two cells per thread; otherwise one copy per pull
-  // (the one-cell kernel's box copies would spill beside an item's descriptor)
+  // is): the two-role kernel, where it is faster on noise fields and on one-fluid
+  // regions; otherwise one copy per pull (the one-cell kernel's box copies would
+  // spill beside an item's descriptor).  It needs the work of 16 planes of a 32 x
+  // 8 column per SM, and with component pairs, whose halves it collides one by
+  // one in a one-fluid region, boxes of about 96^3.  One copy per pull against
+  // two roles, us per step on noise (on a droplet), without spheres:
+  //   sum / difference  2 x 64^3 31.1, 32.2 (31.6, 32.6)   4 x 64^3 56.0, 50.5 (55.9, 50.5)
+  //                     1 x 96^3 58.7, 50.3 (58.7, 50.4)   8 of 32^3 .. 64^3 83.4, 75.7 (83.7, 75.9)
+  //   components        4 x 64^3 57.0, 49.6 (62.7, 67.5)   8 of 32^3 .. 64^3 84.9, 73.8 (91.5, 103)
+  //                     4 x 96^3  181,  138 ( 189,  182)   2 x 128^3          227,  178 ( 238, 227)
   bool wide = true;
-  for (const Ctx* c : boxes) wide = wide && c->nx % 4 == 0;
+  long planes = 0;
+  for (const Ctx* c : boxes) {
+    wide = wide && c->nx % 4 == 0;
+    planes += long((c->nx + 31) / 32) * ((c->ny + 7) / 8) * c->nz;
+  }
+  wide = wide && planes > 16 * 148 && (c0.sd || planes >= 3000 * long(boxes.size()));
   return by_storage(c0, [&](auto* tag) -> int {
     using S = std::remove_pointer_t<decltype(tag)>;
     using C = typename Store<S>::C;

@@ -98,3 +98,58 @@ def test_ensemble_after_a_box_stepped_alone():
     ens.close()
     for s in alone:
         s.close()
+
+
+def _spec(edges, spheres):
+    """Boxes of these edges with `spheres` spheres each (none where the edge is not a multiple of 8)."""
+    out = []
+    for i, L in enumerate(edges):
+        n = spheres if L % 8 == 0 else 0
+        c = np.array([[0.25, 0.25, 0.25], [0.75, 0.7, 0.3], [0.02, 0.5, 0.97]]) * L + 0.4 + 0.1 * i
+        out.append((L, c[:n]))
+    return out
+
+
+@pytest.mark.parametrize("storage,edges,spheres", [
+    ("f16sd", (64, 48, 96), 3), ("bf16sd", (64, 64, 64), 0),  # two roles
+    ("f16", (96, 104), 2), ("bf16", (96, 96), 0),             # two roles, component pairs of large boxes
+    ("f16", (48, 64, 96), 2),                                 # component pairs of smaller ones: one copy per pull
+    ("f16sd", (32, 48), 2),                                   # too little work for two roles
+    ("f16sd", (30, 96, 64), 2), ("f16", (96, 110), 0),        # a width that is not a multiple of 4
+])
+def test_every_candidate_of_the_tuner_equals_boxes_alone(storage, edges, spheres):
+    """The tuner steps the boxes with 32 x 8 and 32 x 16 columns and six segment lengths (12 candidates, here of four
+    steps each), whichever it picks then: fields, flags and spheres are those of the boxes stepped alone.  Half of the
+    first box is one fluid, so that both ways through a cell run."""
+    spec = _spec(edges, spheres)
+    params = [_params(L, len(x), storage) for L, x in spec]
+    ens = Ensemble(params)
+    alone = []
+    for i, ((L, x), p) in enumerate(zip(spec, params)):
+        rR, rB = seeded_noise_fields(L, L, L, seed=60 + i)
+        if i == 0:
+            rR[:, :, : L // 2], rB[:, :, : L // 2] = 1.0, 0.0
+        v = np.full_like(x, 0.03)
+        for sim in (ens.boxes[i], None):
+            if sim is None:
+                sim = LBSim(p)
+                alone.append(sim)
+            sim.set_fields(rR, rB)
+            if len(x):
+                sim.set_particles(x, v)
+    ens.tune(trial=2)
+    ens.step(3)  # a captured pair and an eager step with the choice
+    for s in alone:
+        s.step(12 * 4 + 3)
+    for i, s in enumerate(alone):
+        assert ens.boxes[i].status()[0] == 0 and s.status()[0] == 0
+        for fa, fb in zip(ens.boxes[i].get_fields(f64=True), s.get_fields(f64=True)):
+            assert np.isfinite(fa).all() and np.array_equal(fa, fb), i
+        if len(spec[i][1]):
+            assert np.array_equal(ens.boxes[i].get_flags(), s.get_flags()), i
+            pa, pb = ens.boxes[i].get_particles(), s.get_particles()
+            for k in pa:
+                assert np.array_equal(pa[k], pb[k]), (i, k)
+    ens.close()
+    for s in alone:
+        s.close()
