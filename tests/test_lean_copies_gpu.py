@@ -1,11 +1,14 @@
-"""The two ways the single-pass kernel stages 16-bit pulls give the same bits.
+"""The kernels that copy 16-bit pulls as boxes and the one that copies each pull give the same bits.
 
-With 16-bit storage the lean colour-gradient kernel copies the pulls of a plane into shared memory two planes
-ahead of their collision, either as 16-byte granules of one box of rows per direction (the default when nx is
-a multiple of 4; copied by some threads, read by all, ordered by per-slot mbarriers) or as one 4-byte copy per
-pull (each thread copies what it reads).  The arithmetic after the copy is the same, so every stored pair,
-particle record and flag must agree bit for bit between the two, on boxes whose columns wrap in x, y and z, on
-both CTA shapes, with and without spheres, and on every 16-bit storage.
+With 16-bit storage the single-pass colour-gradient step copies the pulls of a plane into shared memory ahead of
+their collision, either as 16-byte granules of one box of rows per direction (the default when nx is a multiple of
+4; copied by some threads, read by all, ordered by per-slot mbarriers) or as one 4-byte copy per pull (each thread
+copies what it reads; lbx_set_lean_copies(ctx, 0)).  Boxes of rows go with two kernels: two cells per thread and two
+roles per CTA for the component and the sum / difference pairs without spheres, one cell per thread with spheres and
+for the predicted split.  Component pairs whose automatic segments have one or two planes take one copy per pull
+either way, so the comparisons set the segment length.  Each cell's arithmetic is rounded alike in all of them, so
+every stored pair, particle record and flag must agree bit for bit, on boxes whose columns wrap in x, y and z, on both
+CTA shapes, with and without spheres, and on every 16-bit storage.
 """
 import numpy as np
 import pytest
@@ -77,14 +80,14 @@ def test_moving_spheres_copies_bit_identical(storage, n):
         assert np.array_equal(ra[k], rb[k]), k
 
 
-def _half_plain_run(storage, copies, cta, plain, nx=72, ny=20, nz=24, steps=6):
+def _half_plain_run(storage, copies, cta, plain, nx=72, ny=20, nz=24, steps=6, **more):
     """A box whose cells with x < plain hold one fluid at rest density (no colour gradient there)."""
     rR, rB = seeded_noise_fields(nx, ny, nz, seed=9)
     rR[:, :, :plain] = 1.0
     rB[:, :, :plain] = 0.0
-    g = LBSim(make_params(nx, ny, nz, model="cg", storage=storage, sigma=0.02, beta=0.7))
+    g = LBSim(make_params(nx, ny, nz, model="cg", storage=storage, sigma=0.02, beta=0.7, **more))
     g.set_lean_copies(copies)
-    g.set_lean_shape(cta, 0)
+    g.set_lean_shape(cta, 7)  # segments in which a warp meets such cells plane after plane
     g.set_fields(rR, rB)
     g.step(steps)
     out = g.get_pops()
@@ -102,6 +105,16 @@ def test_cells_without_a_gradient(storage, cta, plain):
         assert np.isfinite(p).all() and np.array_equal(p, q)
 
 
+@pytest.mark.parametrize("storage", ["f16", "bf16", "f16sd", "bf16sd"])
+@pytest.mark.parametrize("shape,cta,zlen", [((64, 16, 24), 1, 6), ((32, 32, 72), 0, 24), ((132, 20, 30), 0, 11)])
+def test_fluid_long_segments(storage, shape, cta, zlen):
+    """Segments that go round the three stage slots several times, on both CTA shapes."""
+    (pa, fa, sa), (pb, fb, sb) = (_fluid_run(shape, storage, m, cta, zlen, 6) for m in (1, 0))
+    assert sa == 0 and sb == 0
+    for a, b in zip(pa + fa, pb + fb):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("storage", ["f16", "bf16", "f16sd"])
 @pytest.mark.parametrize("shape", [(12, 12, 12), (8, 12, 12), (48, 48, 48), (52, 52, 52)])
 def test_small_boxes_take_either_kernel(storage, shape):
@@ -111,3 +124,12 @@ def test_small_boxes_take_either_kernel(storage, shape):
     assert sa == 0 and sb == 0
     for a, b in zip(pa + fa, pb + fb):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("storage", ["f16", "bf16", "f16sd", "bf16sd", "f16sdp"])
+@pytest.mark.parametrize("cta,plain", [(0, 40), (1, 40), (0, 0)])
+def test_two_viscosities(storage, cta, plain):
+    """tauR != tauB: each cell forms its own relaxation rate, in one-fluid cells and in mixed ones."""
+    a, b = (_half_plain_run(storage, m, cta, plain, tauR=1.0, tauB=0.8) for m in (1, 0))
+    for p, q in zip(a, b):
+        assert np.isfinite(p).all() and np.array_equal(p, q)
