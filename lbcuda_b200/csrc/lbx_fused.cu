@@ -31,9 +31,10 @@
 // (PART) also copies each cell's flag words and side phase field with its
 // pulls and collides only fluid cells.
 //
-// 16-bit boxes without spheres and the ensemble run the same march with two
-// cells per thread and two roles per CTA (phase_column2 and
-// collide_column2 below); the results are the same bits.
+// 16-bit component and sum / difference pairs on widths that are multiples of 4,
+// without spheres or in an ensemble, run the same march with two cells per thread
+// and two roles per CTA (phase_column2 and collide_column2 below; launch_lean2
+// and ensemble_launch have the rules); the results are the same bits.
 #include "lbx_device.cuh"
 #include "lbx_roles.h"
 
@@ -1442,15 +1443,14 @@ __device__ __forceinline__ void recolour2(const LeanConst<float>& K, const Relax
 template <bool SD, typename I, typename O>
 __device__ __forceinline__ void bgk2(const LeanConst<float>& K, const Relaxed2& X, V2 rA, V2 rB, I&& in, O&& out) {
   const float(&sh)[2][3] = SD ? K.ssd : K.s;
-  const V2 omm = v_sub(v2(1.f), X.omega);
   const V2 oA = p_mul(X.omega, rA), oB = p_mul(X.omega, rB);
   const V2 uu[3] = {X.u, X.v, X.w};
   auto one = [&](int l, V2 A) {
     const int k = wclass(l);
     V2 a, b;
     in(l, a, b);
-    out(l, p_fma(a, omm, p_fma(p_mul(oA, v2(K.w[k])), A, p_mul(X.omega, v2(-sh[0][k])))),
-        p_fma(b, omm, p_fma(p_mul(oB, v2(K.w[k])), A, p_mul(X.omega, v2(-sh[1][k])))));
+    out(l, p_fma(a, X.omm, p_fma(p_mul(oA, v2(K.w[k])), A, p_mul(X.omega, v2(-sh[0][k])))),
+        p_fma(b, X.omm, p_fma(p_mul(oB, v2(K.w[k])), A, p_mul(X.omega, v2(-sh[1][k])))));
   };
   one(0, X.c0);
 #pragma unroll
@@ -1791,8 +1791,7 @@ __device__ __forceinline__ void collide_column2(const S* __restrict__ A, S* __re
     };
     if (on0 || on1)
       recolour2<SD>(K, X, Ss, rRc, rBc, px, py, pz, psq, [&](int l, V2 a, V2 b) { store2(l, a, b, on0, on1); });
-    // cells without a colour gradient: the BGK result per component; solid
-    // cells: the plain pull
+    // cells without a colour gradient: the BGK result per component
     const bool off0 = col0 && !on0, off1 = col1 && !on1;
     was_off = __any_sync(0xffffffffu, off0 || off1);
     if (off0 || off1) {
@@ -1835,12 +1834,12 @@ __device__ __forceinline__ void collide_registers() {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kCollideRegs));
 }
 
-template <typename S, int TY, bool PART, bool SD>
+template <typename S, int TY, bool SD>
 __global__ void __launch_bounds__(32 * TY, TY == 8 ? 2 : 1)
     k_cg_lean2(const S* __restrict__ A, S* __restrict__ B, Geom g, LeanConst<float> K, int zlen,
-               unsigned long long* err, int64_t step, LeanPart<float> PT, const int4* __restrict__ plan) {
+               unsigned long long* err, int64_t step, const int4* __restrict__ plan) {
   extern __shared__ __align__(16) unsigned char lean_smem[];
-  using M = Col2<S, TY, PART>;
+  using M = Col2<S, TY, false>;
   M::init(lean_smem);
   __syncthreads();
   // the column and z-segment of this CTA: from the grid (equal segments) or
@@ -1856,11 +1855,11 @@ __global__ void __launch_bounds__(32 * TY, TY == 8 ? 2 : 1)
   if (threadIdx.x >= M::NT) {
     phase_registers();
     PhaseSync sy;
-    phase_column2<S, TY, PART, SD>(A, g, K, x0, y0, z0, z1, err, step, PT, lean_smem, sy);
+    phase_column2<S, TY, false, SD>(A, g, K, x0, y0, z0, z1, err, step, LeanPart<float>{}, lean_smem, sy);
   } else {
     collide_registers();
     SlotSeq sy;
-    collide_column2<S, TY, PART, SD>(A, B, g, K, x0, y0, z0, z1, err, step, PART && PT.fnew != nullptr, lean_smem, sy);
+    collide_column2<S, TY, false, SD>(A, B, g, K, x0, y0, z0, z1, err, step, false, lean_smem, sy);
   }
 }
 
@@ -2140,7 +2139,7 @@ static int launch_lean2(Ctx& c, int zlen_override) {
   using M = Col2<S, TY, false>;
   static unsigned long long done = 0;
   static int per_sm[64] = {0}, sms[64] = {0};
-  auto* kernel = k_cg_lean2<S, TY, false, SD>;
+  auto* kernel = k_cg_lean2<S, TY, SD>;
   int rc = allow_smem(kernel, M::BYTES, done);
   if (rc) return rc;
   int dev = 0;
@@ -2174,7 +2173,7 @@ static int launch_lean2(Ctx& c, int zlen_override) {
   }
   if (plan) grid = dim3(unsigned(nplan), 1, 1);
   kernel<<<grid, 2 * M::NT, M::BYTES, c.stream>>>((const S*)c.pops[c.cur], (S*)c.pops[1 - c.cur], geom(c),
-                                              make_lean<float>(c), zlen, c.d_err, c.step + 1, LeanPart<float>{}, plan);
+                                              make_lean<float>(c), zlen, c.d_err, c.step + 1, plan);
   return 0;
 }
 
@@ -2185,11 +2184,19 @@ static int launch_lean(Ctx& c, int zlen_override, LeanPart<typename Store<S>::C>
     // spheres (721 us of the colloid step against 695 at 256^3 with 1280
     // spheres: flags and solid cells lengthen both roles) and with the
     // predicted split (86.6 against 84.3 us at FP16 128^3: a window read per
-    // direction in the collision's chain)
+    // direction in the collision's chain).  One-cell box kernel against two roles,
+    // us per step on noise, on a droplet in its first 24 steps and after 180
+    // (cells without a gradient hold their slot or are pulled again):
+    //   sum / difference  64^3 18.6, 16.7   18.7, 16.7   18.7, 16.8
+    //                    128^3 80.8, 76.8   80.6, 76.8   81.3, 82.6
+    //                    256^3  593,  541    593,  541    640,  600
+    //   FP16 components   64^3 18.7, 16.7   20.7, 21.0   20.7, 20.7
+    //                    128^3 83.2, 77.9    100,  101    104,  104
+    //                    256^3  607,  550    689,  698    693,  698
     if constexpr (PART || SDP) {
       if (use_boxes(c, PART)) return launch_lean_as<S, TX, TY, MINB, PART, SD, SDP, true>(c, zlen_override, pt);
     } else {
-      static const bool fit = roles_fit(k_cg_lean2<S, TY, false, SD>);
+      static const bool fit = roles_fit(k_cg_lean2<S, TY, SD>);
       if (fit && use_boxes(c)) return launch_lean2<S, TY, MINB, SD>(c, zlen_override);
     }
   }
