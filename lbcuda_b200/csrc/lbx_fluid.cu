@@ -19,8 +19,9 @@
 // The colour-gradient collision needs the phase field of all 26 neighbours at
 // the same time level.  Two schedules are provided:
 //   two-pass: k_cg_phi (pull + densities -> phi) then k_cg_collide (the
-//   kernel-level entries, and lbx_set_schedule(ctx, 0) of the single-density
-//   D3Q19 model; two densities and D3Q27 step in one pass, k_cg_march);
+//   kernel-level entries, lbx_set_schedule(ctx, 0) of the single-density D3Q19
+//   model, and two densities and D3Q27 where single_pass() says so; otherwise
+//   those fuse both passes into k_cg_march);
 //   single-pass: k_cg_fused, where each CTA owns a (BX x BY) column of cells
 //   and marches it along z, computing the phase field of its own cells and of
 //   a one-cell ring around the column from the pulled populations into a
@@ -330,14 +331,16 @@ __global__ void __launch_bounds__(TX* TY) k_cg_fused(const S* __restrict__ A, S*
 // column of w x h cells along z over one segment.  Per plane it sums the pulls
 // of plane z+1 for its cells and the ring around them into densities and writes
 // their phase field (DD: and the densities) into a four-plane shared window,
-// then pulls plane z again (from L1 / L2, where the sums left it), takes the
+// then pulls plane z again (from L2, where the sums left it), takes the
 // gradients from the window, collides and stores.  The helpers and their order
 // are those of k_cg_phi and k_cg_collide, so the results are theirs bit for bit.
 // Bound: the chain of a plane (pull, sum, barrier, pull, collide): 5.0 us for a
 // CTA alone on its SM, 6.4 us with two, at FP32 with two densities, whatever
 // the cells do.  So the time follows the planes per resident CTA, and the
-// column's shape and the segments decide (march_plan); columns of 32 x 8 on
-// every box took 43 us a step at 65 x 57 x 49, 22 of 24 columns being partial.
+// column's shape and the segments decide (march_plan).  Per step, new droplet
+// [noise], two passes against one: two densities FP32 64^3 38, 39 us [45, 35],
+// 65 x 57 x 49 38, 32 [44, 29], 128^3 248, 210 [302, 243]; D3Q27 FP32 96^3 139, 120
+// [170, 133].  Floors at the copy rate: 99 us at 128^3, 59 us at 96^3.
 // ---------------------------------------------------------------------------
 template <typename S> struct Pair2;  // the two components of a direction and cell as one word
 template <> struct Pair2<float> { using R = float2; };
@@ -399,7 +402,7 @@ __global__ void __launch_bounds__(March<typename Store<S>::C>::NT, sizeof(typena
   // densities and phase field of cell (px, py) of plane p into its window slot
   auto fill = [&](int px, int py, int p, int slot, bool check) {
     Nbr b;
-    make_nbr(g, px, py, wrapc(p, g.nz), b);
+    make_nbr(g, px, py, p < 0 ? p + g.nz : (p >= g.nz ? p - g.nz : p), b);  // -1 <= p <= nz
     C fR[QQ], fB[QQ];
     pull_pairs<QQ>(A, g, b, sh, fR, fB);
     C rR = sum_q<QQ>(fR), rB = sum_q<QQ>(fB);
