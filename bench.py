@@ -34,12 +34,11 @@ L = 128
 SEED = 1
 SIGMA, BETA = 0.02, 0.7
 LB_PER_STEP = 500
-# DRAM bytes (read + write) of one k_cg_lean launch at 128^3, from the ncu
-# captures summarised in profiles/ (None where no capture of that storage)
-# DRAM read + write bytes of one launch of the fluid kernel at 128^3 (ncu
-# dram__bytes_read.sum + dram__bytes_write.sum, the captures summarised in
-# profiles/k_cg_lean_*_128cube.md); measured, so they change with the kernel
-TRAFFIC = {"f16": 370.1e6, "f16sd": 368.9e6, "f16sdp": 393.7e6, "f32": 622.6e6}
+# Kernel of the spinodal step and its DRAM bytes (read + write) of one launch at
+# 128^3, from ncu dram__bytes_read.sum + dram__bytes_write.sum (the captures
+# summarised in profiles/); measured, so they change with the kernel
+KERNEL = {"f16": "k_cg_lean2", "f16sd": "k_cg_lean2", "f16sdp": "k_cg_lean", "f32": "k_cg_lean"}
+TRAFFIC = {"f16": 376.1e6, "f16sd": 375.9e6, "f16sdp": 393.7e6, "f32": 622.6e6}
 BYTES_PER_CELL = {"f16": 160, "bf16": 160, "f16sd": 160, "bf16sd": 160, "f16sdp": 160, "bf16sdp": 160, "f32": 312,
                   "f64": 616}  # algorithmic bytes per cell-step
 MINIMAL_BYTES = {"f16": 152, "bf16": 152, "f16sd": 152, "f16sdp": 160, "f32": 304, "f64": 608}  # bytes the kernel must move
@@ -781,7 +780,7 @@ def main():
         achieved = alg / (per_launch_ms * 1e-3) / 1e9
         return {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                 "traffic": TRAFFIC.get(storage), "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, "
-                "one launch at 128^3 (profiles/)", "peak_kind": peak_kind, "kernel": "k_cg_lean",
+                "one launch at 128^3 (profiles/)", "peak_kind": peak_kind, "kernel": KERNEL.get(storage, "k_cg_lean"),
                 "bytes_per_cell": BYTES_PER_CELL[storage],
                 "kernel_us_per_launch": per_launch_ms * 1e3,
                 "minimal_bytes_frac": MINIMAL_BYTES[storage] * cells / (per_launch_ms * 1e-3) / 1e9 / hbm}

@@ -335,16 +335,20 @@ int lbx_get_stream(void* ctx, void** stream);
 /* Colour-gradient schedule: 2 = lean single-pass kernel (default), 1 = the
  * first single-pass kernel, 0 = two passes (phase field, then collision).
  * The two-density and D3Q27 models take 0 only (other values: LBX_ERR_ARG);
- * without spheres lbx_step fuses its two passes into one, bit for bit equal.
+ * without spheres lbx_step fuses its two passes into one where that is faster,
+ * bit for bit equal.
  * The reference prints Mlup/s from CUDA events around the step loop
  * (main.CUF:274-292); these are the hooks the benchmark uses for the same. */
 int lbx_set_schedule(void* ctx, int32_t fused);
 /* Lean single-pass kernel shape: 0 = 32x8 cells per CTA, 1 = 32x16; zlen =
- * lattice planes per z-segment (0 = automatic). */
+ * lattice planes per z-segment (0 = automatic), also of the fused step of the
+ * two-density and D3Q27 models. */
 int lbx_set_lean_shape(void* ctx, int32_t shape, int32_t zlen);
-/* How the lean kernel stages 16-bit pulls in shared memory: 1 = 16-byte
- * granules of a box of rows per direction (default; used when nx is a
- * multiple of 4), 0 = one 4-byte copy per pull.  Both give the same bits. */
+/* How 16-bit pulls reach shared memory: 1 = 16-byte granules of a box of rows per
+ * direction (default; used when nx is a multiple of 4, except for component pairs
+ * in small boxes), 0 = one 4-byte copy per pull.  With 1, boxes without spheres
+ * run a kernel of two cells per thread (not the predicted split).  All give the
+ * same bits. */
 int lbx_set_lean_copies(void* ctx, int32_t mode);
 /* Enqueue nsteps steps bracketed by CUDA events on the context stream and
  * wait: total device ms, and the summed duration / launch count of the

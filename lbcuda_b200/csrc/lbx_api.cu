@@ -199,7 +199,7 @@ int lbx_create(const lbx_params* p, void** out) {
   c->n = n;
   c->ncomp = (p->model == LBX_MODEL_BGK) ? 1 : 2;
   c->q = d3q27 ? lbx::Q27 : lbx::Q;
-  // the DIFFDENS collision and the D3Q27 lattice run on the two-pass schedule only
+  // the DIFFDENS collision and the D3Q27 lattice: schedule 0 only
   if (two_dens || d3q27) c->fused = 0;
   c->storage = p->storage;
   c->sd = sd;
@@ -467,8 +467,9 @@ const char* lbx_error_string(int code) {
 }
 
 /* ---- measurement hooks used by the benchmark --------------------------- */
-/* Select the colour-gradient schedule: 1 = single-pass fused kernel (default),
- * 0 = two passes (phase field, then collision). */
+/* Select the colour-gradient schedule: 2 = lean single-pass kernel (default), 1 =
+ * the first single-pass kernel, 0 = two passes (phase field, then collision; the
+ * two-density and D3Q27 models fuse them where that is faster). */
 int lbx_set_schedule(void* ctx, int32_t fused) {
   Ctx* c = as_ctx(ctx);
   if (!c) return LBX_ERR_ARG;
@@ -481,7 +482,7 @@ int lbx_set_schedule(void* ctx, int32_t fused) {
 }
 
 /* Shape of the lean single-pass kernel: shape 0 = 32x8 cells per CTA, 1 =
- * 32x16; zlen = planes per z-segment (0 = automatic). */
+ * 32x16; zlen = planes per z-segment (0 = automatic), also of k_cg_march. */
 int lbx_set_lean_shape(void* ctx, int32_t shape, int32_t zlen) {
   Ctx* c = as_ctx(ctx);
   if (!c || shape < 0 || shape > 1 || zlen < 0) return LBX_ERR_ARG;
@@ -566,7 +567,8 @@ int lbx_get_stream(void* ctx, void** stream) {
   return 0;
 }
 
-/* Staging of the lean kernel's 16-bit pulls: 1 = box granules, 0 = one copy per pull. */
+/* Copies of 16-bit pulls: 1 = box granules (two-role or one-cell kernel), 0 = one
+ * copy per pull. */
 int lbx_set_lean_copies(void* ctx, int32_t mode) {
   Ctx* c = as_ctx(ctx);
   if (!c || mode < 0 || mode > 1) return LBX_ERR_ARG;

@@ -110,7 +110,7 @@ __device__ __forceinline__ void fma1(float4& s, float a, float4 b) {
   s.w = fmaf(a, b.w, s.w);
 }
 
-// activation and its derivative from one exponential (the values of silu and dsilu)
+// activation and its derivative
 __device__ __forceinline__ void act(float z, float* A, float* S) {
   *A = silu(z);
   *S = dsilu(z);

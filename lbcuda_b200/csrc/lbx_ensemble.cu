@@ -5,15 +5,15 @@
 // closure are set and read with the ordinary entry points.  A step of the
 // ensemble forks from the ensemble stream to the stream of every box with
 // spheres, runs that box's sphere pre-kernels there, joins, launches ONE
-// persistent colour-gradient kernel for the fluid of all boxes
-// (k_cg_lean2_multi for 16-bit storage, else k_cg_lean_multi: CTAs take (box,
-// column, z-segment) work items, longest first) on the ensemble stream, then forks and joins again around the sphere
-// post-kernels.  The boxes' small sphere kernels thus run side by side
-// instead of one after the other.  Two consecutive steps (the ping-pong
-// parity) are captured once into a CUDA graph (the forks become parallel
-// branches) and replayed, so the host issues one graph launch per two steps.  lbx_ensemble_tune times the
-// fused fluid kernel of each candidate CTA shape and z-segment length on the
-// boxes themselves and keeps the fastest.
+// persistent colour-gradient kernel for the fluid of all boxes (CTAs take (box,
+// column, z-segment) work items, longest first; k_cg_lean2_multi or
+// k_cg_lean_multi, ensemble_launch has the rule) on the ensemble stream, then
+// forks and joins again around the sphere post-kernels.  The boxes' small sphere
+// kernels thus run side by side instead of one after the other.  Two consecutive
+// steps (the ping-pong parity) are captured once into a CUDA graph (the forks
+// become parallel branches) and replayed, so the host issues one graph launch per
+// two steps.  lbx_ensemble_tune times the fused fluid kernel of each candidate CTA
+// shape and z-segment length on the boxes themselves and keeps the fastest.
 #include <algorithm>
 #include <new>
 #include <vector>

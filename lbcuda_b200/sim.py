@@ -116,14 +116,15 @@ class LBSim:
         check(self._L.lbx_sync(self._h), "lbx_sync")
 
     def set_schedule(self, fused):
-        """0 = two passes, 1 = first single-pass kernel, 2 = lean single-pass kernel (default)."""
+        """0 = two passes (two-density and D3Q27 models, which take 0 only: fused where that is faster), 1 = first
+        single-pass kernel, 2 = lean single-pass kernel (default)."""
         check(self._L.lbx_set_schedule(self._h, int(fused)), "lbx_set_schedule")
 
     def set_lean_shape(self, shape, zlen=0):
         check(self._L.lbx_set_lean_shape(self._h, int(shape), int(zlen)), "lbx_set_lean_shape")
 
     def set_lean_copies(self, mode):
-        """16-bit pulls of the lean kernel: 1 = 16-byte box granules (default), 0 = one copy per pull."""
+        """16-bit pulls: 1 = 16-byte box granules (default), 0 = one copy per pull; the same bits."""
         check(self._L.lbx_set_lean_copies(self._h, int(mode)), "lbx_set_lean_copies")
 
     def time_steps(self, n, kernel_timing=True):

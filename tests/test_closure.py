@@ -2,7 +2,7 @@
 use inside the particle step, and a small end-to-end gain check.
 
 The closure has no counterpart in the reference; the numpy reference
-(oracle/M.py) is itself checked against finite differences.
+(oracle/mlp_ref.py) is itself checked against finite differences.
 Tolerances: GPU gradient vs numpy 1e-4 relative (FP32 vs FP64), inference
 1e-5 relative to the output scale.
 """

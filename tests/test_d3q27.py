@@ -1,7 +1,7 @@
 """The D3Q27 lattice (the reference's D3Q27 build, dimensions_m.CUF:117-198).
 
 CPU checks of the oracle restatement on 27 directions, and (gpu) parity of
-the two-pass kernels against it: FP32 storage 1e-5 relative (velocity as
+the step against it: FP32 storage 1e-5 relative (velocity as
 relative L2), FP64 1e-12.
 """
 import numpy as np

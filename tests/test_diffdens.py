@@ -1,8 +1,8 @@
 """Two fluid densities (the reference's DIFFDENS build, LBX_MODEL_CG_DIFFDENS).
 
 CPU checks of the oracle restatement (kernels_fluid_CG.CUF:40-49, 163-177,
-539-819; SetConstants main.CUF:1047-1083) and GPU parity of the two-pass
-kernels against it.  Tolerances as for the single-density model: FP32
+539-819; SetConstants main.CUF:1047-1083) and GPU parity of the step
+against it.  Tolerances as for the single-density model: FP32
 storage 1e-5 relative (max norm; velocity as relative L2), FP64 1e-12.
 """
 import numpy as np
@@ -154,7 +154,7 @@ def test_diffdens_arguments():
         LBSim(dd_params(16, 1.0, 0.0))
     g = LBSim(dd_params(16, 1.0, 0.5))
     with pytest.raises(LBXError):
-        g.set_schedule(2)  # the two-density collision runs on the two-pass schedule
+        g.set_schedule(2)  # the two-density collision takes schedule 0 only
     g.set_schedule(0)
     g.close()
 
