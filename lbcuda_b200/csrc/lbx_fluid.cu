@@ -847,20 +847,20 @@ int fluid_bgk(Ctx& c) {
 
 // Whether a step of the two-density and D3Q27 models takes k_cg_march.  FP32 and
 // FP64 pairs, both models at once, and FP16 with two densities: always (1.3 times
-// as fast as two passes on average; down to 0.91 in the first steps of a droplet,
-// FP64 with 56^3 cells, and 0.97 to 0.98 in FP32 around 44^3 to 64^3).  The other
-// 16-bit models: not between small boxes, where it saves a launch, and a million
-// cells.  There the two passes gain more from the cells of one fluid, which they
-// do not recolour, and a box of two fluids is mostly such cells once it has
-// separated.  Two passes against one, us per step on a droplet [on noise]:
+// as fast as two passes on average; down to 0.9 in the first steps of a droplet in
+// FP64 with 56^3 cells or 120 x 50 x 40, 0.99 in FP32 at 64^3).  The other 16-bit
+// models: not between small boxes, where it saves a launch, and 800,000 cells.
+// There the two passes gain more from the cells of one fluid, which they do not
+// recolour, and a box of two fluids is mostly such cells once it has separated.
+// Two passes against one, us per step on a droplet [on noise]:
 //   D3Q27 FP16      40^3 21.3, 18.8 [24.7, 20.1]   64^3 37.2, 40.2 [45.2, 39.6]
-//                   88^3 90.7, 96.2 [116, 98]     100^3  149,  127 [194, 137]
+//                   88^3 90.7, 96.2 [116, 98]      96^3  109,  105 [138, 109]
 //   2 densities     40^3 20.6, 17.8 [23.7, 18.6]   64^3 33.5, 37.9 [39.2, 35.4]
 //   BF16            88^3 81.5, 87.6 [97.7, 84.2]  100^3  141,  119 [174, 115]
 static bool single_pass(const Ctx& c) {
   const bool both = two_densities(c) && c.q == Q27;
   if (c.elem != 2 || both || (two_densities(c) && c.storage == LBX_STORE_F16)) return true;
-  return c.n <= 64000 || c.n >= 1000000;
+  return c.n <= 64000 || c.n >= 800000;
 }
 
 int fluid_step(Ctx& c) {
